@@ -39,6 +39,7 @@ struct Batch {
     int n = 0;
     long long total_rays = 0, out_len = 0;
     int spec_len = 0, max_nf = 1;
+    bool fixed = false;  // every image is one the fixed-point geodesic covers (FxGeo::ok)
     size_t h2d_bytes = 0;
     std::vector<raptor::DevImage> host;
     std::vector<int> spec_img, spec_f;
@@ -92,7 +93,9 @@ int build_dev_image(raptor_gpu_ctx* ctx, const raptor_image_desc& d, raptor::Dev
 int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs, Batch& b);
 // form: RAPTOR_PREC_FP64, RAPTOR_PREC_MIXED or RAPTOR_PREC_MIXED_DF
 // pool: the FP64 form's sample-pool kernel (ray_kernel_pool) instead of ray_kernel
-RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool = true);
+// fixed: the fixed-point geodesic's kernels (FP64 and mixed forms; Batch::fixed)
+RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed);
+RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool);
 RayLaunchFn pick_ray_kernel_df(int nf, const void** fn);
 LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form);
 LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp);

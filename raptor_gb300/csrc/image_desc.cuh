@@ -4,6 +4,7 @@
 // pixels, set_units grmhd.c:17-33, set_constants utilities.c:17-26).
 #pragma once
 #include "checked.cuh"
+#include "fixed_geodesic.cuh"
 #include "kerr_mks.cuh"
 
 namespace raptor {
@@ -96,6 +97,8 @@ struct DevImage {
     // the device after each upload, read by the FP64 and mixed kernels'
     // start_ray
     MksPoint cam_point;
+    // constants of the fixed-point geodesic (fixed_geodesic.cuh)
+    FxGeo fx;
 };
 
 // Per-step record of one traced ray (the analogue of the reference's GEOD

@@ -141,10 +141,12 @@ extern "C" int raptor_gpu_render_noalloc(int device, const double* d_cells, cons
     int h_map[2 * RAPTOR_NOALLOC_MAX_IMAGES * RAPTOR_MAX_FREQS];
     long long rays = 0, outlen = 0;
     int nspec = 0, max_nf = 1;
+    bool fixed = true;
     for (int k = 0; k < n_imgs; ++k) {
         raptor_image_desc d = imgs[k];
         d.grid = 0;
         if (build_dev_image(&shim, d, h_desc[k]) != RAPTOR_OK) return RAPTOR_ERR_INVALID;
+        fixed = fixed && h_desc[k].fx.ok;
         h_desc[k].ray_begin = rays;
         h_desc[k].out_offset = outlen;
         rays += (long long)d.width * d.height;
@@ -180,7 +182,7 @@ extern "C" int raptor_gpu_render_noalloc(int device, const double* d_cells, cons
     // the FP64 form's default kernel and launch shape, as raptor_gpu_render
     // picks them without tuning
     const void* fnp = nullptr;
-    RayLaunchFn fn = pick_ray_kernel(max_nf, RAPTOR_PREC_FP64, &fnp);
+    RayLaunchFn fn = pick_ray_kernel(max_nf, RAPTOR_PREC_FP64, &fnp, true, fixed);
     int occ = 1, sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fnp, kRayMaxBlock, 0) != cudaSuccess)

@@ -75,6 +75,37 @@ static bool finite_all(std::initializer_list<double> v) {
     return true;
 }
 
+// x 2^q as an integer, for |x| 2^q below 2^63 (clamped there)
+static long long to_fixed(double x, int q) {
+    const double v = std::ldexp(x, q);
+    return v >= 0x1p63 ? 0x7fffffffffffffffll : v <= -0x1p63 ? -0x7fffffffffffffffll : std::llrint(v);
+}
+// a b 2^-s, rounded down
+static long long mul_fixed(long long a, long long b, int s) { return (long long)(((__int128)a * b) >> s); }
+
+// Constants of the fixed-point geodesic (fixed_geodesic.cuh), and whether the
+// image is one it covers: r = exp(x1), theta(x2) with a derivative well away
+// from 0, and a step parameter whose steps move ln r by a tenth at most.
+static FxGeo fixed_geo(const raptor_grid_geom& g, const DevImage& im, double stepsize) {
+    FxGeo f{};
+    f.ok = g.R0 == 0.0 && g.hslope >= 0.2 && g.hslope <= 1.8 && stepsize >= 1e-7 && stepsize <= 0.1;
+    if (!f.ok) return f;
+    f.a = to_fixed(g.a, 62);
+    f.a2 = mul_fixed(f.a, f.a, 62);
+    const long long omh = (1ll << 62) - to_fixed(g.hslope, 62);  // 1 - h, Q62
+    f.tc = mul_fixed(omh, 2935890503282001226ll, 64);            // 1 / (4 pi) in Q65
+    f.ph = mul_fixed(omh, 7244019458077122842ll, 63);            // pi in Q61
+    f.th2 = -mul_fixed(omh, 5689439577989151081ll, 62);          // 2 pi^2 in Q58
+    f.eps = to_fixed(stepsize, 64);
+    f.startx1 = to_fixed(im.startx1, 59);
+    f.stopx1 = to_fixed(im.stopx1, 59);
+    f.startx2 = to_fixed(im.startx2, 62);
+    f.stopx2 = to_fixed(im.stopx2, 62);
+    f.ln_inner = to_fixed(log(im.cutoff_inner), 59);
+    f.ln_outer = to_fixed(log(kCutoffOuter), 59);
+    return f;
+}
+
 int build_dev_image(raptor_gpu_ctx* ctx, const raptor_image_desc& d, DevImage& im) {
     if (d.grid < 0 || d.grid >= RAPTOR_MAX_GRIDS || !ctx->grids[d.grid].used)
         return ctx_fail(ctx, RAPTOR_ERR_INVALID, "image refers to grid %d, which is not uploaded", d.grid);
@@ -218,6 +249,7 @@ int build_dev_image(raptor_gpu_ctx* ctx, const raptor_image_desc& d, DevImage& i
     im.stopx2_df = df_const(im.stopx2);
     im.idx1_df = df_const(im.idx1);
     im.idx2_df = df_const(im.idx2);
+    im.fx = fixed_geo(g, im, d.stepsize);
     return RAPTOR_OK;
 }
 
@@ -433,9 +465,10 @@ static void launch_ray_pool(const LaunchShape& ls, cudaStream_t st, const DevIma
     else ray_kernel_pool<NF><<<ls.grid, ls.block, 0, st>>>(imgs, n, b, e, ctr, out, ls.refill);
 }
 
-RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool) {
+RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed) {
     if (form == RAPTOR_PREC_MIXED_DF) return pick_ray_kernel_df(nf, fn);
     const bool mixed = form == RAPTOR_PREC_MIXED;
+    if (fixed) return pick_ray_kernel_fx(nf, mixed, fn, pool);
     // one instantiation per frequency-count bucket so tau/I stay in registers
 #define PICK(NF)                                                        \
     if (nf <= NF) {                                                     \
@@ -459,12 +492,14 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
     b.out_len = 0;
     b.spec_len = 0;
     b.max_nf = 1;
+    b.fixed = true;
     b.host.resize(n_imgs);
     b.spec_img.clear();
     b.spec_f.clear();
     for (int k = 0; k < n_imgs; ++k) {
         int rc = build_dev_image(ctx, imgs[k], b.host[k]);
         if (rc) return rc;
+        b.fixed = b.fixed && b.host[k].fx.ok;
         b.host[k].ray_begin = b.total_rays;
         b.host[k].out_offset = b.out_len;
         b.total_rays += (long long)imgs[k].width * imgs[k].height;
@@ -652,7 +687,7 @@ static int render_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n
     if (rb > b.total_rays) return ctx_fail(ctx, RAPTOR_ERR_INVALID, "ray range starts past the batch");
     const int form = precision;
     const void* fnp = nullptr;
-    RayLaunchFn fn = pick_ray_kernel(b.max_nf, form, &fnp, !ctx->opt.no_sample_pool);
+    RayLaunchFn fn = pick_ray_kernel(b.max_nf, form, &fnp, !ctx->opt.no_sample_pool, b.fixed);
     LaunchShape ls = choose_shape(ctx, b, form, fn, fnp);
     bool replayed = false;
     if (ctx->opt.use_graph && rb == 0 && re == b.total_rays) {
@@ -718,7 +753,7 @@ extern "C" int raptor_gpu_trace_ray(raptor_gpu_ctx* ctx, const raptor_image_desc
     if (rc) return rc;
     CK(cudaMemsetAsync(ctx->d_trace, 0, bytes, ctx->stream));
     const void* fnp = nullptr;
-    RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, false);
+    RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, false, false);  // the trace kernels step in FP64
     LaunchShape ls = default_shape(ctx, fnp, precision);
     ls.grid = 1;
     ls.block = 32;

@@ -269,8 +269,29 @@ __device__ __forceinline__ double null_drift(const MksPoint& p, const Geo& g, co
     return fabs(kk) / (k0 * k0);
 }
 
+// Launch bounds: blocks of at most 128 threads, at least kRayMinBlocks
+// resident per SM, so the register budget (<= 168 per thread at 3) keeps
+// 12 warps per SM to hide FP64 latency.
+#ifndef RAPTOR_RAY_MIN_BLOCKS
+#define RAPTOR_RAY_MIN_BLOCKS 3
+#endif
+constexpr int kRayMaxBlock = 128;
+constexpr int kRayMinBlocks = RAPTOR_RAY_MIN_BLOCKS;
+
+// The pooled kernel's: 2 gives 192 registers a thread and 8 warps, 1 %
+// faster at 1024x1024 than 3 (168 registers, 12 warps; 4 blocks spill).
+#ifndef RAPTOR_POOL_MIN_BLOCKS
+#define RAPTOR_POOL_MIN_BLOCKS 2
+#endif
+constexpr int kPoolMinBlocks = RAPTOR_POOL_MIN_BLOCKS;
+
+// A ray of the FP64 geodesic.  The kernels below are templates over the
+// state type: this one, or the fixed-point one of ray_fixed.cuh.
 template <int NF, bool MIXED>
 struct RayState {
+    static constexpr int kTicketRows = 16;  // of the sample pool (PoolLayout)
+    static constexpr int kRayBlocks = kRayMinBlocks, kPoolBlocks = kPoolMinBlocks;
+    static constexpr bool kLockstep = false;  // the pooled kernel's warps step together (a block barrier per step)
     double y[8];
     MksPoint p;
     double beta, thdot_prev;
@@ -300,15 +321,6 @@ __device__ __forceinline__ void trace_record(const TraceSpec& tr, const RayState
     r[14] = s.stop;
     r[15] = 0.0;
 }
-
-// Launch bounds: blocks of at most 128 threads, at least kRayMinBlocks
-// resident per SM, so the register budget (<= 168 per thread at 3) keeps
-// 12 warps per SM to hide FP64 latency.
-#ifndef RAPTOR_RAY_MIN_BLOCKS
-#define RAPTOR_RAY_MIN_BLOCKS 3
-#endif
-constexpr int kRayMaxBlock = 128;
-constexpr int kRayMinBlocks = RAPTOR_RAY_MIN_BLOCKS;
 
 // Per-launch statistics of the ray kernels, folded over the warp and added
 // to the counters buffer by one lane per warp.
@@ -403,7 +415,7 @@ __device__ __forceinline__ void finish_ray(const DevImage& im, const RayState<NF
 // event: 0 stepped outside the sampling region, 1 inside it (sample due),
 // 3 escaped outward (integrator.c:271-272), -1 the while-condition ended the
 // ray before the step.  dl is the step taken.
-template <int NF, bool MIXED, bool TPhi = true>
+template <bool TPhi, int NF, bool MIXED>
 __device__ __forceinline__ int advance_ray(const DevImage& im, RayState<NF, MIXED>& s, double& dl) {
     // while-condition of integrator.c:228-229 (r = exp(x1), no R0)
     const double r = s.p.rp;
@@ -421,14 +433,21 @@ __device__ __forceinline__ int advance_ray(const DevImage& im, RayState<NF, MIXE
     return 0;
 }
 
+// The in-place sample of a ray that has stepped by dl inside the region.
+template <int NF, bool MIXED>
+__device__ __forceinline__ bool sample_ray(const DevImage& im, RayState<NF, MIXED>& s, double dl) {
+    if constexpr (MIXED) return rt_sample_fp32<NF>(im, s.y, s.p, fabs(dl), s.tf, s.tc, s.If, s.Ic);
+    else return rt_sample_fp64<NF>(im, s.y, s.p, fabs(dl), s.tau, s.I);
+}
+
 // TRACE: the per-step trace kernel (t and phi integrated, records written)
-template <int NF, bool MIXED, bool TRACE>
-__global__ void __launch_bounds__(kRayMaxBlock, kRayMinBlocks)
+template <int NF, bool MIXED, bool TRACE, class S = RayState<NF, MIXED>>
+__global__ void __launch_bounds__(kRayMaxBlock, S::kRayBlocks)
     ray_kernel(const DevImage* __restrict__ imgs, int n_imgs, long long ray_begin, long long ray_end,
                unsigned long long* __restrict__ counters, double* __restrict__ out, int refill_interval,
                TraceSpec tr) {
     const int lane = threadIdx.x & 31;
-    RayState<NF, MIXED> s;
+    S s;
     bool active = false, live = true;
     const DevImage* im = imgs;
     RayCounters c;
@@ -448,7 +467,9 @@ __global__ void __launch_bounds__(kRayMaxBlock, kRayMinBlocks)
                     if (ri) {
                         im = ri;
                         active = true;
-                        if (TRACE && rid == tr.ray) trace_record<NF, MIXED>(tr, s, 0.0, 0);
+                        if constexpr (TRACE) {
+                            if (rid == tr.ray) trace_record(tr, s, 0.0, 0);
+                        }
                     }
                 } else {
                     live = false;
@@ -459,17 +480,17 @@ __global__ void __launch_bounds__(kRayMaxBlock, kRayMinBlocks)
         if (active) {
             for (int it = 0; it < refill_interval; ++it) {
                 double dl = 0.0;
-                int event = advance_ray<NF, MIXED, TRACE>(*im, s, dl);
+                int event = advance_ray<TRACE>(*im, s, dl);
                 const bool done = event == -1 || event == 3;
                 if (event == 1) {
                     ++c.rt_calls;
-                    bool sampled;
-                    if constexpr (MIXED) sampled = rt_sample_fp32<NF>(*im, s.y, s.p, fabs(dl), s.tf, s.tc, s.If, s.Ic);
-                    else sampled = rt_sample_fp64<NF>(*im, s.y, s.p, fabs(dl), s.tau, s.I);
+                    const bool sampled = sample_ray(*im, s, dl);
                     c.rt_samples += sampled ? 1 : 0;
                     event = sampled ? 2 : 1;
                 }
-                if (TRACE && event != -1 && s.rid == tr.ray) trace_record<NF, MIXED>(tr, s, dl, event);
+                if constexpr (TRACE) {
+                    if (event != -1 && s.rid == tr.ray) trace_record(tr, s, dl, event);
+                }
                 if (done) {
                     finish_ray(*im, s, out, c);
                     active = false;
@@ -499,12 +520,6 @@ __global__ void __launch_bounds__(kRayMaxBlock, kRayMinBlocks)
 // the two kernels' arithmetic alike (the 1-, 2- and 4-frequency
 // instantiations), and to rounding elsewhere.
 constexpr int kPoolCap = 64;  // ring entries per warp: up to 31 waiting + 32 appended in one step
-// at least this many 128-thread blocks per SM: 2 gives 192 registers a
-// thread and 8 warps, 1 % faster at 1024x1024 than 3 (168 registers, 12
-// warps; 4 blocks spill)
-#ifndef RAPTOR_POOL_MIN_BLOCKS
-#define RAPTOR_POOL_MIN_BLOCKS 2
-#endif
 #ifndef RAPTOR_POOL_DRAIN_WAIT
 #define RAPTOR_POOL_DRAIN_WAIT 4
 #endif
@@ -562,12 +577,12 @@ struct TicketRing {
     __device__ __forceinline__ void ray_ended() { wait = 0; }
 };
 
-template <int NF>
+template <int NF, int Rows>
 struct PoolLayout {
-    // ticket fields, one row of kPoolCap doubles each: 0 |dl|, 1-2 x1 x2,
-    // 3-6 k^mu, 7-15 the point (r, s, c, Sigma, theta', iS, irp, ithp, isn);
-    // evaluated, rows 1..NF hold dtau and NF+1..2NF j / nu_p^2
-    static constexpr int kIn = 16;
+    // ticket fields, one row of kPoolCap doubles each: 0 |dl|, the others the
+    // state type's (put_ticket); evaluated, rows 1..NF hold dtau and
+    // NF+1..2NF j / nu_p^2
+    static constexpr int kIn = Rows;
     static constexpr int kOut = 1 + 2 * NF;
     static constexpr int kFields = kIn > kOut ? kIn : kOut;
     // + the next-ticket links and image indices (two ints per entry), and in
@@ -575,11 +590,57 @@ struct PoolLayout {
     static constexpr int kWarpDoubles = kFields * kPoolCap + kPoolCap + (kChecked ? kPoolCap / 2 : 0);
 };
 
+// A ticket's sample inputs after |dl|: rows 1-2 x1 x2, 3-6 k^mu, 7-15 the
+// point (r, s, c, Sigma, theta', iS, irp, ithp, isn).
 template <int NF>
-__global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_POOL_MIN_BLOCKS)
+__device__ __forceinline__ void put_ticket(const RayState<NF, false>& s, double* e) {
+    constexpr int C = kPoolCap;
+    e[1 * C] = s.y[1];
+    e[2 * C] = s.y[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[(3 + i) * C] = s.y[4 + i];
+    e[7 * C] = s.p.r;
+    e[8 * C] = s.p.s;
+    e[9 * C] = s.p.c;
+    e[10 * C] = s.p.Sg;
+    e[11 * C] = s.p.thp;
+    e[12 * C] = s.p.iS;
+    e[13 * C] = s.p.irp;
+    e[14 * C] = s.p.ithp;
+    e[15 * C] = s.p.isn;
+}
+template <class S>
+struct TicketReader;
+template <int NF>
+struct TicketReader<RayState<NF, false>> {
+    static __device__ __forceinline__ void get(const DevImage&, const double* e, double y[8], MksPoint& mp) {
+        constexpr int C = kPoolCap;
+        y[0] = 0.0;
+        y[1] = e[1 * C];
+        y[2] = e[2 * C];
+        y[3] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[4 + i] = e[(3 + i) * C];
+        mp.rp = 0.0;  // the metric does not read rp, s2x, c2x
+        mp.s2x = 0.0;
+        mp.c2x = 0.0;
+        mp.r = e[7 * C];
+        mp.s = e[8 * C];
+        mp.c = e[9 * C];
+        mp.Sg = e[10 * C];
+        mp.thp = e[11 * C];
+        mp.iS = e[12 * C];
+        mp.irp = e[13 * C];
+        mp.ithp = e[14 * C];
+        mp.isn = e[15 * C];
+    }
+};
+
+template <int NF, class S = RayState<NF, false>>
+__global__ void __launch_bounds__(kRayMaxBlock, S::kPoolBlocks)
     ray_kernel_pool(const DevImage* __restrict__ imgs, int n_imgs, long long ray_begin, long long ray_end,
                     unsigned long long* __restrict__ counters, double* __restrict__ out, int refill_interval) {
-    using L = PoolLayout<NF>;
+    using L = PoolLayout<NF, S::kTicketRows>;
     constexpr int C = kPoolCap;
     __shared__ double pool_mem[(kRayMaxBlock / 32) * L::kWarpDoubles];
     const int lane = threadIdx.x & 31;
@@ -588,7 +649,7 @@ __global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_POOL_MIN_BLOCKS)
     int* const timg = nxt + C;
     int* const towner = timg + C;  // checked build only
     unsigned long long* const cw = imgs[0].check_word;
-    RayState<NF, false> s;
+    S s;
     int mode = 0;  // 0 idle, 1 stepping, 2 ended with tickets outstanding
     bool live = true;
     TicketRing ring;
@@ -618,14 +679,14 @@ __global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_POOL_MIN_BLOCKS)
                 }
             }
         }
-        if (!__any_sync(kFull, mode != 0)) break;
+        if (!(S::kLockstep ? __syncthreads_or(mode != 0) : __any_sync(kFull, mode != 0))) break;
         ++since_refill;
 
         // one geodesic step per stepping lane; a step inside the region appends a ticket
         bool want = false;
         double dl = 0.0;
         if (mode == 1) {
-            const int event = advance_ray<NF, false, false>(*im, s, dl);
+            const int event = advance_ray<false>(*im, s, dl);
             if (event == 1) {
                 ++c.rt_calls;
                 want = true;
@@ -644,19 +705,7 @@ __global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_POOL_MIN_BLOCKS)
         if (t >= 0) {
             double* e = fld + t;
             e[0] = fabs(dl);
-            e[1 * C] = s.y[1];
-            e[2 * C] = s.y[2];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) e[(3 + i) * C] = s.y[4 + i];
-            e[7 * C] = s.p.r;
-            e[8 * C] = s.p.s;
-            e[9 * C] = s.p.c;
-            e[10 * C] = s.p.Sg;
-            e[11 * C] = s.p.thp;
-            e[12 * C] = s.p.iS;
-            e[13 * C] = s.p.irp;
-            e[14 * C] = s.p.ithp;
-            e[15 * C] = s.p.isn;
+            put_ticket(s, e);
             timg[t] = s.img;
         }
 
@@ -669,26 +718,10 @@ __global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_POOL_MIN_BLOCKS)
                 double* e = fld + te;
                 double y[8];
                 MksPoint mp;
-                y[0] = 0.0;
-                y[1] = e[1 * C];
-                y[2] = e[2 * C];
-                y[3] = 0.0;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) y[4 + i] = e[(3 + i) * C];
-                mp.rp = 0.0;  // the metric does not read rp, s2x, c2x
-                mp.s2x = 0.0;
-                mp.c2x = 0.0;
-                mp.r = e[7 * C];
-                mp.s = e[8 * C];
-                mp.c = e[9 * C];
-                mp.Sg = e[10 * C];
-                mp.thp = e[11 * C];
-                mp.iS = e[12 * C];
-                mp.irp = e[13 * C];
-                mp.ithp = e[14 * C];
-                mp.isn = e[15 * C];
+                const DevImage& ti = imgs[timg[te]];
+                TicketReader<S>::get(ti, e, y, mp);
                 double dtau[NF], jn[NF];
-                const bool ok = rt_terms_fp64<NF>(imgs[timg[te]], y, mp, e[0], dtau, jn);
+                const bool ok = rt_terms_fp64<NF>(ti, y, mp, e[0], dtau, jn);
                 c.rt_samples += ok ? 1 : 0;
 #pragma unroll
                 for (int f = 0; f < NF; ++f) {

@@ -504,18 +504,24 @@ __device__ __forceinline__ MetricT<float> metric_f32(const PointF32& q, float a,
 // warp's non-sampling lanes idle; the roundings are f32_of's, on the
 // integer pipes, for the same reason).
 template <int NF>
+__device__ __forceinline__ bool rt_sample_fp32_at(const DevImage& im, const PointF32& q, double x1, double x2,
+                                                  const float k[4], double adl, float (&tau)[NF],
+                                                  float (&tauc)[NF], float (&I)[NF], float (&Ic)[NF]) {
+    const MetricT<float> g = metric_f32(q, im.geo_df.a.hi, im.geo_df.a2.hi, im.geo_df.R0.hi);
+    const CellCoef cc = cell_coef(im, x1, x2);
+    float v[8];
+    interp_prims(im.cells32, im.n2, cc, v);
+    return rt_sample_fp32_core<NF>(im, g, v, k, [&](int f) { return f32_of(adl * im.rg_over_nu[f]); }, tau,
+                                   tauc, I, Ic);
+}
+template <int NF>
 __device__ __forceinline__ bool rt_sample_fp32(const DevImage& im, const double y[8], const MksPoint& p,
                                                double adl, float (&tau)[NF], float (&tauc)[NF],
                                                float (&I)[NF], float (&Ic)[NF]) {
     const PointF32 q{f32_of(p.r),  f32_of(p.s),   f32_of(p.iS),   f32_of(p.thp),
                      f32_of(p.Sg), f32_of(p.irp), f32_of(p.ithp), f32_of(p.isn)};
-    const MetricT<float> g = metric_f32(q, im.geo_df.a.hi, im.geo_df.a2.hi, im.geo_df.R0.hi);
-    const CellCoef cc = cell_coef(im, y[1], y[2]);
-    float v[8];
-    interp_prims(im.cells32, im.n2, cc, v);
     const float k[4] = {f32_of(y[4]), f32_of(y[5]), f32_of(y[6]), f32_of(y[7])};
-    return rt_sample_fp32_core<NF>(im, g, v, k, [&](int f) { return f32_of(adl * im.rg_over_nu[f]); }, tau,
-                                   tauc, I, Ic);
+    return rt_sample_fp32_at<NF>(im, q, y[1], y[2], k, adl, tau, tauc, I, Ic);
 }
 
 }  // namespace raptor

@@ -34,7 +34,8 @@ std::string signature(const raptor_gpu_ctx* ctx, const Batch& b, int form) {
                        : form == RAPTOR_PREC_MIXED  ? "mixed"
                        : ctx->opt.no_sample_pool    ? "fp64_inplace"
                                                     : "fp64";
-    snprintf(k, sizeof k, "%s|%s|nf%d|2^%d", ctx->device_name, name, b.max_nf, size_class);
+    const char* geo = b.fixed && form != RAPTOR_PREC_MIXED_DF ? "_fx" : "";
+    snprintf(k, sizeof k, "%s|%s%s|nf%d|2^%d", ctx->device_name, name, geo, b.max_nf, size_class);
     std::string s(k);
     for (char& c : s)
         if (c == ' ') c = '_';

@@ -980,7 +980,7 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
         unsigned long long fwd_ctr[kCtrCount] = {};
         if (!one_pass) {
             const void* fnp = nullptr;
-            RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, !ctx->opt.no_sample_pool);
+            RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, !ctx->opt.no_sample_pool, b.fixed);
             LaunchShape ls = choose_shape(ctx, b, precision, fn, fnp);
             rc = enqueue_render(ctx, b, precision, rb, re, ls, fn, true);
             if (rc) return rc;
