@@ -46,6 +46,7 @@
 
 #ifdef __CUDACC__
 #define FX_HD __device__ __forceinline__
+#define FX_MEMBER __device__ __forceinline__
 #define FX_TABLE(name, n) __device__ const longlong2 name[n]
 #else
 #include <cstdint>
@@ -53,6 +54,7 @@ struct longlong2 {
     long long x, y;
 };
 #define FX_HD static inline
+#define FX_MEMBER inline
 #define FX_TABLE(name, n) static const longlong2 name[n]
 #endif
 
@@ -312,10 +314,18 @@ FX_HD fx fx_isigma(const FxGeo& g, const FxPoint& p, int n, fx& a2w2, fx& s2, fx
     return fx_recip(sg);                                // 2/sigma in Q61, the integer of 1/sigma in Q62
 }
 
+// The terms of a stage's right-hand side and the point, for a tangent of it.
+struct FxTerms {
+    fx w, ww, wt2, wt3, a2w2, s2, sg, isg, rho, dl, isg2, isg3, beta, bw, gam, aw, sc, thi, t, tw, as2;
+    fx P, R1, S, H, X0, Y, Q, RK, kap2, kap3, mu, s0, s1;
+    fx sg2, wr2, rww, F1, F2, z, A, g2, G, B, F3, D;
+    fx E0, E1, E2a, E2b, E3a, E3b;
+};
+
 // K' = E: E0, E1 in Q60, E2 = E2a + E2b 2^(2u-ks) and E3 = E3a - 2 E3b 2^ks
 // with E2a, E2b, E3a in Q57 and E3b in Q58.  v2, v3 in Q59.
 FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, int n, int p, int u, fx v2, fx v3,
-                  fx& E0, fx& E1, fx& E2a, fx& E2b, fx& E3a, fx& E3b) {
+                  FxTerms& o) {
     fx a2w2, s2, sg;  // Q62, Q62, Q61
     const fx isg = fx_isigma(g, q, n, a2w2, s2, sg);
     const fx w = q.w >> n;                         // Q62
@@ -335,7 +345,8 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     const fx t = mulk<2>(mulk<2>(a2w2, sc), thi);  // Q60
     const fx tw = mulk<2>(mulk<2>(t, isg), w);     // t w/sigma, Q60
 
-    const fx P = fx_scale(mulk<4>(mulk<2>(g.a, s2), v3), u - n);  // Q61
+    const fx as2 = mulk<2>(g.a, s2);               // Q62
+    const fx P = fx_shl(mulk<4>(as2, v3) >> n, u);  // Q61
     const fx R1 = mulk<2>(q.r, k1);                // Q60
     const fx S = (k0 >> 1) + R1;                   // K0 + R1, Q60
     const fx H = sqrk<2>(S);                       // Q58
@@ -350,43 +361,58 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     {
         FxAcc s = fx_mul(ww, X0);
         s = fx_mac(s, sg2w, Y);
-        s = fx_mac(s, sg + (w >> 1), mulk<3>(R1, k1));  // Q61 x (Q60 x Q61 -> Q60)
-        FxAcc e = fx_mul(bw, -fx_sum<1>(s));       // Q62 x Q58; doubled below
-        E0 = fx_sum<5>(e) + mulk<6>(mulk<5>(tw, v2), S - (P >> 1)) + (fx_shl(mu, 2) >> n);
+        o.RK = mulk<3>(R1, k1);                    // Q60
+        s = fx_mac(s, sg + (w >> 1), o.RK);        // Q61 x Q60
+        o.s0 = fx_sum<1>(s);                       // Q58
+        const FxAcc e = fx_mul(bw, -o.s0);         // Q62 x Q58; doubled below
+        o.E0 = fx_sum<5>(e) + mulk<6>(mulk<5>(tw, v2), S - (P >> 1)) + (fx_shl(mu, 2) >> n);
     }
     {
         FxAcc s = fx_mul(wt2, mulk<3>(dl, X0));            // Q62 x Q59
         s = fx_mac(s, mulk<3>(q.w, dl - sg), Y);           // 2 w~ (delta - sigma) in Q61 x Q60
         s = fx_mac(s, dl - fx_shl(sg, 1), Q);              // -(2 sigma - delta) Q61 x Q60
-        FxAcc e = fx_mul(bw, -fx_sum<1>(s));               // Q62 x Q58
+        o.s1 = fx_sum<1>(s);                               // Q58
+        FxAcc e = fx_mul(bw, -o.s1);                       // Q62 x Q58
         e = fx_mac(e, mulk<2>(isg, q.w), -mulk<1>(k1, P));  // 2 K1 P in Q58
         e = fx_mac(e, t, mulk<5>(k1, v2));                 // Q60 x 2 K1 V2 in Q60
         e = fx_mac(e, dl, mu);                             // Q61 x Q59
-        E1 = fx_sum<4>(e) - Q;
+        o.E1 = fx_sum<4>(e) - Q;
     }
     const fx sg2 = sqrk<2>(sg);                    // Q60
     const fx wr2 = mulk<2>(w, rho);                // 2 w rho in Q60
     const fx kv23 = mulk<4>(k2, v3);               // Q60
     {
-        const fx F1 = fx_sum<1>(fx_mac(fx_mul(sg2 + wr2, k1), mulk<2>(rho, ww), k0));  // Q58
+        o.rww = mulk<2>(rho, ww);                                                      // Q61
+        const fx F1 = fx_sum<1>(fx_mac(fx_mul(sg2 + wr2, k1), o.rww, k0));             // Q58
         const fx F2 = fx_sum<3>(fx_mac(fx_mul(dl, sg2), wr2, rho));                    // Q60
         const fx z = mulk<3>(mulk<2>(sc, isg3), q.ithp);                               // Q62
-        FxAcc e = fx_mul(mulk<3>(a2w2, wt3) >> p, mulk<1>(z, H));  // 2 a^2 w^2 w~^3 in Q61 x Q57
+        o.A = mulk<3>(a2w2, wt3) >> p;                              // 2 a^2 w^2 w~^3 2^-p in Q61
+        FxAcc e = fx_mul(o.A, mulk<1>(z, H));                       // x Q57
         const fx g2 = mulk<2>(g.th2, mulk<3>(q.s2x, q.ithp));       // th''/th', Q58
         e = fx_mac(e, (t >> 2) - g2, mulk<4>(k2, v2));              // Q58 x Q60
-        E2a = fx_sum<3>(e) - mulk<1>(mulk<1>(isg, k1), k2);         // 2 () in Q57 is ()'s integer in Q58
+        o.E2a = fx_sum<3>(e) - mulk<1>(mulk<1>(isg, k1), k2);         // 2 () in Q57 is ()'s integer in Q58
+        o.F1 = F1; o.F2 = F2; o.z = z; o.g2 = g2;
         const fx G = mulk<2>(F2, v3) - (mulk<2>(aw, F1) >> u);      // Q57 (2 a w F1 in Q57)
-        E2b = mulk<2>(fx_shl(z, q.ks), mulk<3>(k3, G));             // Q62 x Q57
+        o.G = G;
+        o.E2b = mulk<2>(fx_shl(z, q.ks), mulk<3>(k3, G));             // Q62 x Q57
     }
     {
-        FxAcc e = fx_mul(mulk<2>(mulk<2>(g.a, bw), wt3) >> (p + u), mulk<1>(k0, P) - H);  // Q61 x -(H - 2 K0 P) Q58
-        E3a = fx_sum<2>(e) - mulk<1>(mulk<1>(gam, k3), k1 - mulk<1>(q.w, P))   // Q60 x (2 K1 - w~ P) Q60
+        o.B = mulk<2>(mulk<2>(g.a, bw), wt3) >> (p + u);                       // Q61
+        const FxAcc e = fx_mul(o.B, mulk<1>(k0, P) - H);                       // x -(H - 2 K0 P) Q58
+        o.E3a = fx_sum<2>(e) - mulk<1>(mulk<1>(gam, k3), k1 - mulk<1>(q.w, P))   // Q60 x (2 K1 - w~ P) Q60
               + (mulk<1>(aw, mulk<3>(kap2, mulk<2>(thi, k2))) >> u)            // Q62 x Q58
               - mulk<3>(tw, kv23);                                             // Q60 x Q60, times 4
         const fx F3 = fx_sum<2>(fx_mac(fx_mul(ww, k0), sg2w, k1));             // Q60
         const fx D = kv23 - (mulk<2>(mulk<2>(aw, isg2), mulk<3>(k2, F3)) >> u);  // Q60
-        E3b = mulk<3>(mulk<2>(mulk<2>(q.c, q.isn), q.thp), D);                 // cot th' 2^-ks Q59 x Q60
+        o.E3b = mulk<3>(mulk<2>(mulk<2>(q.c, q.isn), q.thp), D);               // cot th' 2^-ks Q59 x Q60
+        o.F3 = F3;
+        o.D = D;
     }
+    // (terms that nothing reads cost nothing: the function is inlined)
+    o.w = w; o.ww = ww; o.wt2 = wt2; o.wt3 = wt3; o.a2w2 = a2w2; o.s2 = s2; o.sg = sg; o.isg = isg;
+    o.rho = rho; o.dl = dl; o.isg2 = isg2; o.isg3 = isg3; o.beta = beta; o.bw = bw; o.gam = gam; o.aw = aw;
+    o.sc = sc; o.thi = thi; o.t = t; o.tw = tw; o.as2 = as2; o.P = P; o.R1 = R1; o.S = S; o.H = H; o.X0 = X0;
+    o.Y = Y; o.Q = Q; o.kap2 = kap2; o.kap3 = kap3; o.mu = mu; o.sg2 = sg2; o.wr2 = wr2;
 }
 
 FX_HD fx fx_vshift(fx k, int e) { return e > 1 ? fx_shl(k, e - 2) : k >> (2 - e); }  // K 2^e in Q59
@@ -446,11 +472,19 @@ FX_HD bool fx_step_size(const FxGeo& g, const FxState& s, int ks, fx& L) {
 // lambda: the step size, then RK4 or RK2; dl is |d lambda|.  pt is the point
 // at the ray's position on entry and on exit (not formed for a raw state).
 // slow(s) takes the steps that this arithmetic does not cover, leaves s
-// fixed-point again or raw, and returns |d lambda|.
-template <class Slow>
-FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl, Slow slow) {
+// fixed-point again or raw, and returns |d lambda|.  tan follows the steps
+// that it does cover (the adjoint's tangents; FxNoTangent): begin with the
+// step size, stage with each stage's state, commit when the step holds.
+struct FxNoTangent {
+    FX_MEMBER void begin(const FxState&, const FxPoint&, fx) {}
+    FX_MEMBER void stage(int, int, const FxPoint&, const FxTerms&, fx, fx, fx, fx) {}
+    FX_MEMBER void commit() {}
+};
+template <class Slow, class Tangent>
+FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl, Slow slow, Tangent& tan) {
     fx L = 0;
     bool go = fx_step_size(g, s, pt.ks, L);
+    if (go) tan.begin(s, pt, L);
     const int e = s.p - s.n;
     const fx full = -L, half = full >> 1;
     fx x1 = s.x1, x2 = s.x2, k0 = s.k0, k1 = s.k1, k2 = s.k2, k3 = s.k3;
@@ -481,6 +515,7 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
                 s.k1 = k1;
                 s.k2 = k2;
                 s.k3 = k3;
+                tan.commit();
             } else {
                 dl = slow(s);
                 if (s.raw) break;
@@ -496,16 +531,17 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
         if (q == end) break;
         if (go) {
             const fx v2 = fx_vshift(k2, e), v3 = fx_vshift(k3, e);
-            fx E0, E1, E2a, E2b, E3a, E3b;
-            fx_rhs(g, pt, k0, k1, k2, k3, s.n, s.p, s.u, v2, v3, E0, E1, E2a, E2b, E3a, E3b);
+            FxTerms o;
+            fx_rhs(g, pt, k0, k1, k2, k3, s.n, s.p, s.u, v2, v3, o);
+            tan.stage(q, end, pt, o, k0, k1, k2, k3);
             // offsets h f1, h f2, d f3, h f4 (h = d/2): y + d (f1 + 2 f2 + 2 f3 + f4)/6
             // is y + (o1 + 2 o2 + o3 + o4)/3; RK2: h f1, then y + d f2
             const fx h = q == end - 2 + (rk2 ? 1 : 0) ? full : half;
             const fx o1 = mulk<2>(h, k1), o2 = mulk<5>(h, v2);  // Q61, Q62
             const fx hk = fx_shl(h, pt.ks);
-            const fx p0 = mulk<3>(h, E0), p1 = mulk<3>(h, E1);  // Q61
-            const fx p2 = mulk<6>(h, E2a) + (mulk<6>(hk, E2b) >> (2 * (pt.ks - s.u)));
-            const fx p3 = mulk<6>(h, E3a) - mulk<6>(hk, E3b);  // 2 E3b in Q57
+            const fx p0 = mulk<3>(h, o.E0), p1 = mulk<3>(h, o.E1);  // Q61
+            const fx p2 = mulk<6>(h, o.E2a) + (mulk<6>(hk, o.E2b) >> (2 * (pt.ks - s.u)));
+            const fx p3 = mulk<6>(h, o.E3a) - mulk<6>(hk, o.E3b);  // 2 E3b in Q57
             const int two = q == 1 ? 1 : 0;
             a1 += fx_shl(o1, two);
             a2 += fx_shl(o2, two);

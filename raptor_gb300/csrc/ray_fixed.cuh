@@ -25,7 +25,7 @@ __device__ __forceinline__ fx fx_of(double v, int b) { return __double2ll_rn(sca
 
 // Doubles x1, x2, k^mu into c: the fixed-point state where fx_step covers it,
 // else as they are.
-__device__ __noinline__ void fx_encode(const FxGeo& g, const double* y, FxState* c) {
+static __device__ __noinline__ void fx_encode(const FxGeo& g, const double* y, FxState* c) {
     const double x1 = y[0], x2 = y[1];
     bool ok = g.ok && x1 > 0.0 && x1 < 9.7 && x2 > 0.0001220703125 && x2 < 0.9998779296875;
 #pragma unroll
@@ -87,7 +87,7 @@ __device__ __forceinline__ void fx_decode(const FxState& c, double y[6]) {
 
 // One step in FP64 (step_size and rk4_step or rk2_step of ray_kernel.cuh);
 // returns |d lambda|.
-__device__ __noinline__ double fx_slow_step(const DevImage& im, FxState* c) {
+static __device__ __noinline__ double fx_slow_step(const DevImage& im, FxState* c) {
     double d[6];
     fx_decode(*c, d);
     double y[8] = {0.0, d[0], d[1], 0.0, d[2], d[3], d[4], d[5]};
@@ -104,11 +104,11 @@ __device__ __noinline__ double fx_slow_step(const DevImage& im, FxState* c) {
     return fabs(dl);
 }
 
-__device__ __noinline__ void fx_slow_point(const DevImage& im, double x1, double x2, MksPoint* p) {
+static __device__ __noinline__ void fx_slow_point(const DevImage& im, double x1, double x2, MksPoint* p) {
     mks_point(x1, x2, im.geo, *p);
 }
 // the point where a ray starts, once per ray
-__device__ __noinline__ void fx_start_point(const FxGeo& g, const FxState* c, FxPoint* pt) {
+static __device__ __noinline__ void fx_start_point(const FxGeo& g, const FxState* c, FxPoint* pt) {
     fx_point(g, fx_log2r(c->x1) - fx_shl((fx)c->n, 57), c->x2, *pt);
 }
 
@@ -152,6 +152,30 @@ __device__ __forceinline__ void fx_sample_inputs(const DevImage& im, const FxSta
     mp.irp = fx_double(q.w, -62 - c.n);
     mp.ithp = fx_double(q.ithp, -61);
     mp.isn = fx_double(q.isn, q.ks - 61);
+}
+
+// The tests of advance_ray (ray_kernel.cuh) on the fixed-point state, on ln r
+// where that one compares r: within the cut-off radii, the sign of k^2,
+// escaped outward, inside the sampling region.
+__device__ __forceinline__ bool fx_in_range(const DevImage& im, const FxState& c) {
+    if (!c.raw) return c.x1 < im.fx.ln_outer && c.x1 > im.fx.ln_inner;
+    const double r = exp(__longlong_as_double(c.x1));
+    return r < kCutoffOuter && r > im.cutoff_inner;
+}
+__device__ __forceinline__ int fx_theta_sign(const FxState& c) {
+    if (!c.raw) return c.k2 > 0 ? 1 : (c.k2 < 0 ? -1 : 0);
+    const double k2 = __longlong_as_double(c.k2);
+    return k2 > 0.0 ? 1 : (k2 < 0.0 ? -1 : 0);
+}
+__device__ __forceinline__ bool fx_escaped(const DevImage& im, const FxState& c) {
+    if (!c.raw) return c.x1 > im.fx.stopx1 && c.k1 < 0;
+    return __longlong_as_double(c.x1) > im.stopx1 && __longlong_as_double(c.k1) < 0.0;
+}
+__device__ __forceinline__ bool fx_in_grid(const DevImage& im, const FxState& c) {
+    if (!c.raw)
+        return c.x1 < im.fx.stopx1 && c.x1 > im.fx.startx1 && c.x2 > im.fx.startx2 && c.x2 < im.fx.stopx2;
+    const double x1 = __longlong_as_double(c.x1), x2 = __longlong_as_double(c.x2);
+    return x1 < im.stopx1 && x1 > im.startx1 && x2 > im.startx2 && x2 < im.stopx2;
 }
 
 // 4 blocks of 128 threads per SM (128 registers): the kernels wait on
@@ -234,42 +258,27 @@ __device__ __forceinline__ void finish_ray(const DevImage& im, const FxRay<NF, M
     finish_ray<NF, MIXED>(im, r, out, c);
 }
 
-// advance_ray of ray_kernel.cuh on the fixed-point state: the same tests,
-// on ln r where that one compares r.
+// advance_ray of ray_kernel.cuh on the fixed-point state.
 template <bool TPhi, int NF, bool MIXED>
 __device__ __forceinline__ int advance_ray(const DevImage& im, FxRay<NF, MIXED>& s, double& dl) {
     static_assert(!TPhi, "t and phi are not integrated in fixed point");
     FxState& c = s.c;
-    bool on;
-    int th;
-    if (!c.raw) {
-        on = c.x1 < im.fx.ln_outer && c.x1 > im.fx.ln_inner;
-        th = c.k2 > 0 ? 1 : (c.k2 < 0 ? -1 : 0);
-    } else {
-        const double r = exp(__longlong_as_double(c.x1)), k2 = __longlong_as_double(c.k2);
-        on = r < kCutoffOuter && r > im.cutoff_inner;
-        th = k2 > 0.0 ? 1 : (k2 < 0.0 ? -1 : 0);
-    }
-    if (!(on && s.steps < (int)kMaxSteps && !s.stop)) return -1;
+    const int th = fx_theta_sign(c);
+    if (!(fx_in_range(im, c) && s.steps < (int)kMaxSteps && !s.stop)) return -1;
     if (s.thdot_prev * th < 0 && s.steps > 2) s.turns += 1;
     s.thdot_prev = th;
     if ((s.beta < 0.0 && s.turns > kMaxOrder) || (s.beta > 0.0 && s.turns > kMaxOrder + 1)) s.stop = 1;
-    fx_step(im.fx, c, s.pt, im.integrator == 2, dl, [&](FxState& st) {
+    FxNoTangent none;
+    const auto slow = [&](FxState& st) {
         FxState t = st;
         const double d = fx_slow_step(im, &t);
         st = t;
         return d;
-    });
+    };
+    fx_step(im.fx, c, s.pt, im.integrator == 2, dl, slow, none);
     s.steps += 1;
-    if (!c.raw) {
-        if (c.x1 > im.fx.stopx1 && c.k1 < 0) return 3;
-        if (c.x1 < im.fx.stopx1 && c.x1 > im.fx.startx1 && c.x2 > im.fx.startx2 && c.x2 < im.fx.stopx2) return 1;
-        return 0;
-    }
-    const double x1 = __longlong_as_double(c.x1), x2 = __longlong_as_double(c.x2);
-    if (x1 > im.stopx1 && __longlong_as_double(c.k1) < 0.0) return 3;
-    if (x1 < im.stopx1 && x1 > im.startx1 && x2 > im.startx2 && x2 < im.stopx2) return 1;
-    return 0;
+    if (fx_escaped(im, c)) return 3;
+    return fx_in_grid(im, c) ? 1 : 0;
 }
 
 template <int NF, bool MIXED>

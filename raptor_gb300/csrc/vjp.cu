@@ -1003,7 +1003,7 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
         const VjpLaunchFn vfn =
             precision == RAPTOR_PREC_MIXED_DF ? pick_vjp_df(b.max_nf, &kp, kappa, one_pass)
             : precision == RAPTOR_PREC_MIXED
-                ? pick_vjp_mixed(b.max_nf, &kp, kappa, one_pass)
+                ? (b.fixed ? pick_vjp_fx : pick_vjp_mixed)(b.max_nf, &kp, kappa, one_pass)
                 : pick_vjp_fp64(b.max_nf, &kp, !ctx->opt.no_sample_pool, &scratch_rows, kappa, one_pass);
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kp, kVjpBlock, 0));
         const int grid = ctx->num_sms * std::max(occ, 1);

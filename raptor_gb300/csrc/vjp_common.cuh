@@ -145,5 +145,7 @@ using VjpLaunchFn = void (*)(int grid, cudaStream_t st, const DevImage* im, cons
 // adjoints' picker is pick_vjp_fp64, vjp.cu.)
 VjpLaunchFn pick_vjp_df(int nf, const void** fn, bool kappa, bool tape);
 VjpLaunchFn pick_vjp_mixed(int nf, const void** fn, bool kappa, bool tape);
+// the mixed adjoint of the images that the fixed-point geodesic covers (vjp_fx.cu)
+VjpLaunchFn pick_vjp_fx(int nf, const void** fn, bool kappa, bool tape);
 
 }  // namespace raptor
