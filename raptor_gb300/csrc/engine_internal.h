@@ -94,8 +94,9 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
 // form: RAPTOR_PREC_FP64, RAPTOR_PREC_MIXED or RAPTOR_PREC_MIXED_DF
 // pool: the FP64 form's sample-pool kernel (ray_kernel_pool) instead of ray_kernel
 // fixed: the fixed-point geodesic's kernels (FP64 and mixed forms; Batch::fixed)
-RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed);
-RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool);
+// rays: how many the batch has
+RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed, long long rays);
+RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool, long long rays);
 RayLaunchFn pick_ray_kernel_df(int nf, const void** fn);
 LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form);
 LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp);

@@ -323,7 +323,7 @@ struct FxTerms {
 };
 
 // K' = E: E0, E1 in Q60, E2 = E2a + E2b 2^(2u-ks) and E3 = E3a - 2 E3b 2^ks
-// with E2a, E2b, E3a in Q57 and E3b in Q58.  v2, v3 in Q59.
+// with E2a, E2b, E3a in Q57 and E3b in Q58.  v2, v3 in Q58.
 FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, int n, int p, int u, fx v2, fx v3,
                   FxTerms& o) {
     fx a2w2, s2, sg;  // Q62, Q62, Q61
@@ -339,33 +339,35 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     const fx beta = mulk<3>(fx_one(62) - sg, isg3);  // (2 - sigma) Q61: Q62
     const fx bw = mulk<2>(beta, w);                // Q62
     const fx gam = isg - mulk<2>(mulk<2>(a2w2, s2), bw);  // Q62
-    const fx aw = mulk<2>(g.a, w);                 // Q62
+    const fx awt = mulk<2>(g.a, q.w), aw = awt >> n;  // a w~, a w, Q62
     const fx sc = mulk<2>(q.s, q.c);               // Q62
     const fx thi = mulk<2>(q.thp, isg);            // th'/sigma, Q60
     const fx t = mulk<2>(mulk<2>(a2w2, sc), thi);  // Q60
     const fx tw = mulk<2>(mulk<2>(t, isg), w);     // t w/sigma, Q60
 
     const fx as2 = mulk<2>(g.a, s2);               // Q62
-    const fx P = fx_shl(mulk<4>(as2, v3) >> n, u);  // Q61
+    const fx P = fx_shl(mulk<5>(as2, v3) >> n, u);  // Q61
     const fx R1 = mulk<2>(q.r, k1);                // Q60
     const fx S = (k0 >> 1) + R1;                   // K0 + R1, Q60
     const fx H = sqrk<2>(S);                       // Q58
     const fx X0 = mulk<2>(k0, (k0 >> 1) - P);      // Q61 x Q60: Q59 (2P in Q60 is P's integer)
     const fx Y = mulk<2>(k1, k0 - P);              // Q60
     const fx Q = sqrk<2>(k1);                      // Q60
-    const fx kap2 = mulk<5>(q.thp, v2);            // Q60
-    const fx kap3 = fx_shl(mulk<3>(q.s, v3), u);   // Q60
-    const fx mu = fx_sum<2>(fx_mac(fx_mul(isg, sqrk<3>(kap2)), gam, sqrk<3>(kap3)));  // Q59
+    const fx kap2 = mulk<6>(q.thp, v2);            // Q60
+    const fx M2 = mulk<3>(kap2, mulk<6>(thi, v2));  // kap2^2/sigma, Q59
+    const fx kap3 = fx_shl(mulk<4>(q.s, v3), u);   // Q60
+    const fx mu = M2 + mulk<2>(gam, sqrk<3>(kap3));  // Q59
 
     const fx sg2w = sg + w;                        // sigma + 2w, Q61
+    const fx isgk1 = mulk<1>(isg, k1);             // Q60
+    const fx wP = mulk<2>(q.w, P);                 // Q61
     {
         FxAcc s = fx_mul(ww, X0);
         s = fx_mac(s, sg2w, Y);
         o.RK = mulk<3>(R1, k1);                    // Q60
         s = fx_mac(s, sg + (w >> 1), o.RK);        // Q61 x Q60
         o.s0 = fx_sum<1>(s);                       // Q58
-        const FxAcc e = fx_mul(bw, -o.s0);         // Q62 x Q58; doubled below
-        o.E0 = fx_sum<5>(e) + mulk<6>(mulk<5>(tw, v2), S - (P >> 1)) + (fx_shl(mu, 2) >> n);
+        o.E0 = mulk<6>(mulk<6>(tw, v2), S - (P >> 1)) + (fx_shl(mu, 2) >> n) - mulk<5>(bw, o.s0);
     }
     {
         FxAcc s = fx_mul(wt2, mulk<3>(dl, X0));            // Q62 x Q59
@@ -373,14 +375,14 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
         s = fx_mac(s, dl - fx_shl(sg, 1), Q);              // -(2 sigma - delta) Q61 x Q60
         o.s1 = fx_sum<1>(s);                               // Q58
         FxAcc e = fx_mul(bw, -o.s1);                       // Q62 x Q58
-        e = fx_mac(e, mulk<2>(isg, q.w), -mulk<1>(k1, P));  // 2 K1 P in Q58
-        e = fx_mac(e, t, mulk<5>(k1, v2));                 // Q60 x 2 K1 V2 in Q60
+        e = fx_mac(e, isgk1, -wP);                         // Q60 x 2 w~ P in Q60
+        e = fx_mac(e, t, mulk<6>(k1, v2));                 // Q60 x 2 K1 V2 in Q60
         e = fx_mac(e, dl, mu);                             // Q61 x Q59
         o.E1 = fx_sum<4>(e) - Q;
     }
     const fx sg2 = sqrk<2>(sg);                    // Q60
     const fx wr2 = mulk<2>(w, rho);                // 2 w rho in Q60
-    const fx kv23 = mulk<4>(k2, v3);               // Q60
+    const fx kv23 = mulk<5>(k2, v3);               // Q60
     {
         o.rww = mulk<2>(rho, ww);                                                      // Q61
         const fx F1 = fx_sum<1>(fx_mac(fx_mul(sg2 + wr2, k1), o.rww, k0));             // Q58
@@ -389,18 +391,18 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
         o.A = mulk<3>(a2w2, wt3) >> p;                              // 2 a^2 w^2 w~^3 2^-p in Q61
         FxAcc e = fx_mul(o.A, mulk<1>(z, H));                       // x Q57
         const fx g2 = mulk<2>(g.th2, mulk<3>(q.s2x, q.ithp));       // th''/th', Q58
-        e = fx_mac(e, (t >> 2) - g2, mulk<4>(k2, v2));              // Q58 x Q60
-        o.E2a = fx_sum<3>(e) - mulk<1>(mulk<1>(isg, k1), k2);         // 2 () in Q57 is ()'s integer in Q58
+        e = fx_mac(e, (t >> 2) - g2, mulk<5>(k2, v2));              // Q58 x Q60
+        o.E2a = fx_sum<3>(e) - mulk<1>(isgk1, k2);                    // 2 () in Q57 is ()'s integer in Q58
         o.F1 = F1; o.F2 = F2; o.z = z; o.g2 = g2;
-        const fx G = mulk<2>(F2, v3) - (mulk<2>(aw, F1) >> u);      // Q57 (2 a w F1 in Q57)
+        const fx G = mulk<3>(F2, v3) - (mulk<2>(aw, F1) >> u);      // Q57 (2 a w F1 in Q57)
         o.G = G;
         o.E2b = mulk<2>(fx_shl(z, q.ks), mulk<3>(k3, G));             // Q62 x Q57
     }
     {
         o.B = mulk<2>(mulk<2>(g.a, bw), wt3) >> (p + u);                       // Q61
         const FxAcc e = fx_mul(o.B, mulk<1>(k0, P) - H);                       // x -(H - 2 K0 P) Q58
-        o.E3a = fx_sum<2>(e) - mulk<1>(mulk<1>(gam, k3), k1 - mulk<1>(q.w, P))   // Q60 x (2 K1 - w~ P) Q60
-              + (mulk<1>(aw, mulk<3>(kap2, mulk<2>(thi, k2))) >> u)            // Q62 x Q58
+        o.E3a = fx_sum<2>(e) - mulk<1>(mulk<1>(gam, k3), k1 - (wP >> 1))         // Q60 x (2 K1 - w~ P) Q60
+              + (mulk<1>(awt >> p, M2) >> (u + 1))                             // a w kap2 th' K2/sigma: Q62 x Q59
               - mulk<3>(tw, kv23);                                             // Q60 x Q60, times 4
         const fx F3 = fx_sum<2>(fx_mac(fx_mul(ww, k0), sg2w, k1));             // Q60
         const fx D = kv23 - (mulk<2>(mulk<2>(aw, isg2), mulk<3>(k2, F3)) >> u);  // Q60
@@ -415,7 +417,7 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     o.Y = Y; o.Q = Q; o.kap2 = kap2; o.kap3 = kap3; o.mu = mu; o.sg2 = sg2; o.wr2 = wr2;
 }
 
-FX_HD fx fx_vshift(fx k, int e) { return e > 1 ? fx_shl(k, e - 2) : k >> (2 - e); }  // K 2^e in Q59
+FX_HD fx fx_vshift(fx k, int e) { return k >> (3 - e); }  // K 2^e in Q58, e <= 3
 
 // The exponents of a state whose log2 r (Q57) is lr: n from r, then m and p
 // so that the wave vector fills its range.
@@ -459,7 +461,7 @@ FX_HD bool fx_step_size(const FxGeo& g, const FxState& s, int ks, fx& L) {
     const fx m2u = fx_shl(m2, s.u);
     if (((m2 >> 1) >> (61 - s.u)) != 0) return false;
     const fx v2 = fx_abs(fx_vshift(s.k2, e)), v3 = fx_abs(fx_vshift(s.k3, e));
-    const fx d = fx_sum<2>(fx_mac(fx_mul(m2, fx_abs(s.k1) >> 2), m2u, v3)) + v2;  // Q59
+    const fx d = fx_sum<3>(fx_mac(fx_mul(m2, fx_abs(s.k1) >> 3), m2u, v3)) + (v2 << 1);  // Q59
     const int kd = fx_clz((ufx)d) - 2;
     if (kd < 1 || kd > 20) return false;
     const fx y = mulk<1>(mulk<3>(g.eps, m2), fx_recip(fx_shl(d, kd)));  // Q65 x Q61: Q63; L = y 2^(kd-3)
@@ -537,7 +539,7 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
             // offsets h f1, h f2, d f3, h f4 (h = d/2): y + d (f1 + 2 f2 + 2 f3 + f4)/6
             // is y + (o1 + 2 o2 + o3 + o4)/3; RK2: h f1, then y + d f2
             const fx h = q == end - 2 + (rk2 ? 1 : 0) ? full : half;
-            const fx o1 = mulk<2>(h, k1), o2 = mulk<5>(h, v2);  // Q61, Q62
+            const fx o1 = mulk<2>(h, k1), o2 = mulk<6>(h, v2);  // Q61, Q62
             const fx hk = fx_shl(h, pt.ks);
             const fx p0 = mulk<3>(h, o.E0), p1 = mulk<3>(h, o.E1);  // Q61
             const fx p2 = mulk<6>(h, o.E2a) + (mulk<6>(hk, o.E2b) >> (2 * (pt.ks - s.u)));

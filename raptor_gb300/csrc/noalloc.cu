@@ -182,7 +182,7 @@ extern "C" int raptor_gpu_render_noalloc(int device, const double* d_cells, cons
     // the FP64 form's default kernel and launch shape, as raptor_gpu_render
     // picks them without tuning
     const void* fnp = nullptr;
-    RayLaunchFn fn = pick_ray_kernel(max_nf, RAPTOR_PREC_FP64, &fnp, true, fixed);
+    RayLaunchFn fn = pick_ray_kernel(max_nf, RAPTOR_PREC_FP64, &fnp, true, fixed, rays);
     int occ = 1, sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fnp, kRayMaxBlock, 0) != cudaSuccess)

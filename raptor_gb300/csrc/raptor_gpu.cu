@@ -465,10 +465,10 @@ static void launch_ray_pool(const LaunchShape& ls, cudaStream_t st, const DevIma
     else ray_kernel_pool<NF><<<ls.grid, ls.block, 0, st>>>(imgs, n, b, e, ctr, out, ls.refill);
 }
 
-RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed) {
+RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed, long long rays) {
     if (form == RAPTOR_PREC_MIXED_DF) return pick_ray_kernel_df(nf, fn);
     const bool mixed = form == RAPTOR_PREC_MIXED;
-    if (fixed) return pick_ray_kernel_fx(nf, mixed, fn, pool);
+    if (fixed) return pick_ray_kernel_fx(nf, mixed, fn, pool, rays);
     // one instantiation per frequency-count bucket so tau/I stay in registers
 #define PICK(NF)                                                        \
     if (nf <= NF) {                                                     \
@@ -687,7 +687,8 @@ static int render_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n
     if (rb > b.total_rays) return ctx_fail(ctx, RAPTOR_ERR_INVALID, "ray range starts past the batch");
     const int form = precision;
     const void* fnp = nullptr;
-    RayLaunchFn fn = pick_ray_kernel(b.max_nf, form, &fnp, !ctx->opt.no_sample_pool, b.fixed);
+    RayLaunchFn fn = pick_ray_kernel(b.max_nf, form, &fnp, !ctx->opt.no_sample_pool, b.fixed,
+                                     b.total_rays);
     LaunchShape ls = choose_shape(ctx, b, form, fn, fnp);
     bool replayed = false;
     if (ctx->opt.use_graph && rb == 0 && re == b.total_rays) {
@@ -753,7 +754,7 @@ extern "C" int raptor_gpu_trace_ray(raptor_gpu_ctx* ctx, const raptor_image_desc
     if (rc) return rc;
     CK(cudaMemsetAsync(ctx->d_trace, 0, bytes, ctx->stream));
     const void* fnp = nullptr;
-    RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, false, false);  // the trace kernels step in FP64
+    RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, false, false, 1);  // the trace kernels step in FP64
     LaunchShape ls = default_shape(ctx, fnp, precision);
     ls.grid = 1;
     ls.block = 32;

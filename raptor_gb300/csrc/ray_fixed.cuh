@@ -178,30 +178,34 @@ __device__ __forceinline__ bool fx_in_grid(const DevImage& im, const FxState& c)
     return x1 < im.stopx1 && x1 > im.startx1 && x2 > im.startx2 && x2 < im.stopx2;
 }
 
-// 4 blocks of 128 threads per SM (128 registers): the kernels wait on
-// instruction fetch and on the multiply-adds' latency, which more warps hide.
-// 1024x1024, FP64 and mixed: 214 and 128 ms; 3 blocks (168 registers) 229 and
-// 129, 5 (96, spilling) slower.  A barrier per step keeps the four warps of a
-// pooled block on the same code: 214 -> 202 ms.
-constexpr int kFxBlocks = 4;
+// Blocks: 128-thread blocks per SM the kernels are compiled for.  They wait on
+// instruction fetch and on the multiply-adds' latency, which more warps hide,
+// but 4 blocks (128 registers) spill where 3 (168) hardly do.  FP64, one
+// frequency: 1024x1024 198 ms at 4 blocks, 205 at 3, 229 at 2; 800x800 122 and
+// 126; 512x512 59.1 and 57.3; 100x100 15.7 and 14.0: kFxManyRays rays and more
+// take 4.  The mixed kernels take 3 (1024x1024 127 ms either way, 512x512 41.4
+// and 39.3).  5 blocks (96 registers) are slower throughout.
+// A barrier per step (kLockstep) keeps the four warps of a pooled block on the
+// same code: 1024x1024 214 -> 202 ms.
+constexpr long long kFxManyRays = 1ll << 19;
 
-template <int NF, bool MIXED>
+template <int NF, bool MIXED, int Blocks>
 struct FxRay {
     static constexpr int kTicketRows = 15;
-    static constexpr int kRayBlocks = kFxBlocks, kPoolBlocks = kFxBlocks;
+    static constexpr int kRayBlocks = Blocks, kPoolBlocks = Blocks;
     static constexpr bool kLockstep = true;
     FxState c;
     FxPoint pt;  // at c's position (not formed while c is raw)
-    double beta;
+    int bsign;       // sign of the impact parameter beta
     int thdot_prev;  // sign of k^2 at the previous step
     int steps, turns, stop, img, pix;
     double tau[NF], I[NF];
     float tf[NF], tc[NF], If[NF], Ic[NF];
 };
 
-template <int NF, bool MIXED>
+template <int NF, bool MIXED, int Blocks>
 __device__ __forceinline__ const DevImage* start_ray(const DevImage* __restrict__ imgs, int n_imgs, long long rid,
-                                                     FxRay<NF, MIXED>& s) {
+                                                     FxRay<NF, MIXED, Blocks>& s) {
     s.img = find_image(imgs, n_imgs, rid);
     if (!chk(s.img >= 0 && s.img < n_imgs, imgs[0].check_word, kChkImage, s.img)) return nullptr;
     const DevImage* im = imgs + s.img;
@@ -210,7 +214,9 @@ __device__ __forceinline__ const DevImage* start_ray(const DevImage* __restrict_
              kChkPixel, rid))
         return nullptr;
     double y[8];
-    init_photon(*im, camera_of(*im), s.pix % im->width, s.pix / im->width, y, s.beta);
+    double beta;
+    init_photon(*im, camera_of(*im), s.pix % im->width, s.pix / im->width, y, beta);
+    s.bsign = beta < 0.0 ? -1 : (beta > 0.0 ? 1 : 0);
     const double d[6] = {y[1], y[2], y[4], y[5], y[6], y[7]};
     FxState c;
     fx_encode(im->fx, d, &c);
@@ -232,8 +238,8 @@ __device__ __forceinline__ const DevImage* start_ray(const DevImage* __restrict_
     return im;
 }
 
-template <int NF, bool MIXED>
-__device__ __forceinline__ void finish_ray(const DevImage& im, const FxRay<NF, MIXED>& s, double* __restrict__ out,
+template <int NF, bool MIXED, int Blocks>
+__device__ __forceinline__ void finish_ray(const DevImage& im, const FxRay<NF, MIXED, Blocks>& s, double* __restrict__ out,
                                            RayCounters& c) {
     RayState<NF, MIXED> r;  // finish_ray reads of it the position, wave vector, sums and step count
     double d[6];
@@ -259,15 +265,15 @@ __device__ __forceinline__ void finish_ray(const DevImage& im, const FxRay<NF, M
 }
 
 // advance_ray of ray_kernel.cuh on the fixed-point state.
-template <bool TPhi, int NF, bool MIXED>
-__device__ __forceinline__ int advance_ray(const DevImage& im, FxRay<NF, MIXED>& s, double& dl) {
+template <bool TPhi, int NF, bool MIXED, int Blocks>
+__device__ __forceinline__ int advance_ray(const DevImage& im, FxRay<NF, MIXED, Blocks>& s, double& dl) {
     static_assert(!TPhi, "t and phi are not integrated in fixed point");
     FxState& c = s.c;
     const int th = fx_theta_sign(c);
     if (!(fx_in_range(im, c) && s.steps < (int)kMaxSteps && !s.stop)) return -1;
     if (s.thdot_prev * th < 0 && s.steps > 2) s.turns += 1;
     s.thdot_prev = th;
-    if ((s.beta < 0.0 && s.turns > kMaxOrder) || (s.beta > 0.0 && s.turns > kMaxOrder + 1)) s.stop = 1;
+    if ((s.bsign < 0 && s.turns > kMaxOrder) || (s.bsign > 0 && s.turns > kMaxOrder + 1)) s.stop = 1;
     FxNoTangent none;
     const auto slow = [&](FxState& st) {
         FxState t = st;
@@ -281,8 +287,8 @@ __device__ __forceinline__ int advance_ray(const DevImage& im, FxRay<NF, MIXED>&
     return fx_in_grid(im, c) ? 1 : 0;
 }
 
-template <int NF, bool MIXED>
-__device__ __forceinline__ bool sample_ray(const DevImage& im, FxRay<NF, MIXED>& s, double dl) {
+template <int NF, bool MIXED, int Blocks>
+__device__ __forceinline__ bool sample_ray(const DevImage& im, FxRay<NF, MIXED, Blocks>& s, double dl) {
     double y[8];
     MksPoint mp;
     if constexpr (MIXED) {
@@ -310,8 +316,8 @@ __device__ __forceinline__ bool sample_ray(const DevImage& im, FxRay<NF, MIXED>&
 
 // The sample pool's tickets: rows 1-6 the state's words, row 7 its exponents
 // (with the point's ks), rows 8-14 the point.
-template <int NF>
-__device__ __forceinline__ void put_ticket(const FxRay<NF, false>& s, double* e) {
+template <int NF, int Blocks>
+__device__ __forceinline__ void put_ticket(const FxRay<NF, false, Blocks>& s, double* e) {
     constexpr int C = kPoolCap;
     const fx w[6] = {s.c.x1, s.c.x2, s.c.k0, s.c.k1, s.c.k2, s.c.k3};
     const fx q[7] = {s.pt.r, s.pt.w, s.pt.s, s.pt.c, s.pt.thp, s.pt.ithp, s.pt.isn};
@@ -321,8 +327,8 @@ __device__ __forceinline__ void put_ticket(const FxRay<NF, false>& s, double* e)
 #pragma unroll
     for (int i = 0; i < 7; ++i) e[(8 + i) * C] = __longlong_as_double(q[i]);
 }
-template <int NF>
-struct TicketReader<FxRay<NF, false>> {
+template <int NF, int Blocks>
+struct TicketReader<FxRay<NF, false, Blocks>> {
     static __device__ __forceinline__ void get(const DevImage& im, const double* e, double y[8], MksPoint& mp) {
         constexpr int C = kPoolCap;
         FxState c;

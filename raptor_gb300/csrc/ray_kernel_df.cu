@@ -258,8 +258,9 @@ __global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_RAY_DF_MIN_BLOCKS)
             if (lane == leader) base = atomicAdd(&counters[kCtrQueue], (unsigned long long)__popc(need));
             base = __shfl_sync(kFull, base, leader);
             if (!active && live) {
-                const long long rid = ray_begin + (long long)(base + __popc(need & ((1u << lane) - 1u)));
-                if (rid < ray_end) {
+                const unsigned long long idx = base + __popc(need & ((1u << lane) - 1u));
+                if ((long long)idx < ray_end - ray_begin) {
+                    const long long rid = ray_begin + queue_order(idx, ray_end - ray_begin);
                     const DevImage* ri = start_ray_df(imgs, n_imgs, rid, s);
                     if (ri) {
                         im = ri;

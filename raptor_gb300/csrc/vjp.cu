@@ -588,8 +588,9 @@ __global__ void __launch_bounds__(kVjpBlock, 1)
             if (lane == leader) base = atomicAdd(&counters[kCtrQueue], (unsigned long long)__popc(need));
             base = __shfl_sync(kFull, base, leader);
             if (mode == 0 && live) {
-                const long long rid = rr.begin + (long long)(base + __popc(need & ((1u << lane) - 1u)));
-                if (rid < rr.end) {
+                const unsigned long long idx = base + __popc(need & ((1u << lane) - 1u));
+                if ((long long)idx < rr.end - rr.begin) {
+                    const long long rid = rr.begin + queue_order(idx, rr.end - rr.begin);
                     pix = (int)rid;
                     nrec = 0;
                     full = false;
@@ -980,7 +981,8 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
         unsigned long long fwd_ctr[kCtrCount] = {};
         if (!one_pass) {
             const void* fnp = nullptr;
-            RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, !ctx->opt.no_sample_pool, b.fixed);
+            RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, !ctx->opt.no_sample_pool, b.fixed,
+                                             b.total_rays);
             LaunchShape ls = choose_shape(ctx, b, precision, fn, fnp);
             rc = enqueue_render(ctx, b, precision, rb, re, ls, fn, true);
             if (rc) return rc;

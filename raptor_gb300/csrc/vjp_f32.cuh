@@ -387,8 +387,9 @@ __device__ __forceinline__ void vjp_f32_body(const DevImage& im, const CamT<D1>&
             if (lane == leader) base = atomicAdd(&counters[kCtrQueue], (unsigned long long)__popc(need));
             base = __shfl_sync(kFull, base, leader);
             if (!active && live) {
-                const long long rid = rr.begin + (long long)(base + __popc(need & ((1u << lane) - 1u)));
-                if (rid < rr.end) {
+                const unsigned long long idx = base + __popc(need & ((1u << lane) - 1u));
+                if ((long long)idx < rr.end - rr.begin) {
+                    const long long rid = rr.begin + queue_order(idx, rr.end - rr.begin);
                     s.pix = (int)rid;
                     const int px = s.pix % im.width, py = s.pix / im.width;
                     D1 y0[8];
