@@ -11,10 +11,11 @@
 #include "raptor_gpu.h"
 
 // geodesic steps between lane refills of the persistent ray kernels when
-// the caller sets none: 8 for the FP64 and mixed forms (1.3 % faster than
-// every step on the 1024x1024 image), 16 for mixed-DF (2 % faster than 8)
+// the caller sets none: 8 where the geodesic is FP64 (1.3 % faster than every
+// step on the 1024x1024 image), 16 where it is fixed point (1024x1024 FP64
+// 198.8 -> 195.6 ms, mixed 125.5 -> 121.6) or double-float (2 % faster than 8)
 constexpr int kDefaultRefill = 8;
-constexpr int kDefaultRefillDF = 16;
+constexpr int kDefaultRefillFast = 16;
 
 struct LaunchShape {
     int block = 128;   // threads per block
@@ -98,7 +99,7 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
 RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed, long long rays);
 RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool, long long rays);
 RayLaunchFn pick_ray_kernel_df(int nf, const void** fn);
-LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form);
+LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, bool fast);
 LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp);
 int enqueue_render(raptor_gpu_ctx* ctx, const Batch& b, int form, long long rb, long long re,
                    const LaunchShape& ls, RayLaunchFn fn, bool timed, raptor::TraceSpec tr = {-1, nullptr, 0});

@@ -316,13 +316,13 @@ FX_HD fx fx_isigma(const FxGeo& g, const FxPoint& p, int n, fx& a2w2, fx& s2, fx
 
 // The terms of a stage's right-hand side and the point, for a tangent of it.
 struct FxTerms {
-    fx w, ww, wt2, wt3, a2w2, s2, sg, isg, rho, dl, isg2, isg3, beta, bw, gam, aw, sc, thi, t, tw, as2;
+    fx w, ww, wt2, wt3, a2w2, s2, sg, isg, rho, dl, isg2, isg3, beta, gam, aw, sc, thi, t, as2;
     fx P, R1, S, H, X0, Y, Q, RK, kap2, kap3, mu, s0, s1;
     fx sg2, wr2, rww, F1, F2, z, A, g2, G, B, F3, D;
     fx E0, E1, E2a, E2b, E3a, E3b;
 };
 
-// K' = E: E0, E1 in Q60, E2 = E2a + E2b 2^(2u-ks) and E3 = E3a - 2 E3b 2^ks
+// K' = E: E0, E1 in Q60, E2 = E2a + E2b 2^(2u-ks) and E3 = E3a + 2 E3b 2^ks
 // with E2a, E2b, E3a in Q57 and E3b in Q58.  v2, v3 in Q58.
 FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, int n, int p, int u, fx v2, fx v3,
                   FxTerms& o) {
@@ -331,25 +331,26 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     const fx w = q.w >> n;                         // Q62
     const fx ww = mulk<2>(w, q.w);                 // w w~, Q62
     const fx wt2 = sqrk<2>(q.w);                   // w~^2, Q62
-    const fx wt3 = mulk<1>(wt2, q.w);              // w~^3, Q61
+    const fx wt3 = mulk<1>(wt2, q.w) >> p;         // w~^3 2^-p, Q61
     const fx rho = fx_one(61) + (a2w2 >> 1);       // Q61
     const fx dl = rho - w;                         // delta, Q61 (2w in Q61 is w's integer)
     const fx isg2 = sqrk<2>(isg);                  // Q62
     const fx isg3 = mulk<2>(isg2, isg);            // Q62
     const fx beta = mulk<3>(fx_one(62) - sg, isg3);  // (2 - sigma) Q61: Q62
-    const fx bw = mulk<2>(beta, w);                // Q62
-    const fx gam = isg - mulk<2>(mulk<2>(a2w2, s2), bw);  // Q62
+    const fx nw = -w;                              // (negative factors, so that the sums below need no negation)
+    const fx nbw = mulk<2>(beta, nw);              // -beta w, Q62
+    const fx gam = isg + mulk<2>(mulk<2>(a2w2, s2), nbw);  // Q62
     const fx awt = mulk<2>(g.a, q.w), aw = awt >> n;  // a w~, a w, Q62
     const fx sc = mulk<2>(q.s, q.c);               // Q62
     const fx thi = mulk<2>(q.thp, isg);            // th'/sigma, Q60
     const fx t = mulk<2>(mulk<2>(a2w2, sc), thi);  // Q60
-    const fx tw = mulk<2>(mulk<2>(t, isg), w);     // t w/sigma, Q60
+    const fx ntw = mulk<4>(mulk<2>(t, isg), nw);   // -t w/sigma, Q62
 
     const fx as2 = mulk<2>(g.a, s2);               // Q62
     const fx P = fx_shl(mulk<5>(as2, v3) >> n, u);  // Q61
     const fx R1 = mulk<2>(q.r, k1);                // Q60
     const fx S = (k0 >> 1) + R1;                   // K0 + R1, Q60
-    const fx H = sqrk<2>(S);                       // Q58
+    const fx H = sqrk<3>(S);                       // Q59
     const fx X0 = mulk<2>(k0, (k0 >> 1) - P);      // Q61 x Q60: Q59 (2P in Q60 is P's integer)
     const fx Y = mulk<2>(k1, k0 - P);              // Q60
     const fx Q = sqrk<2>(k1);                      // Q60
@@ -359,7 +360,7 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     const fx mu = M2 + mulk<2>(gam, sqrk<3>(kap3));  // Q59
 
     const fx sg2w = sg + w;                        // sigma + 2w, Q61
-    const fx isgk1 = mulk<1>(isg, k1);             // Q60
+    const fx nigk1 = -mulk<1>(isg, k1);            // Q60
     const fx wP = mulk<2>(q.w, P);                 // Q61
     {
         FxAcc s = fx_mul(ww, X0);
@@ -367,15 +368,17 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
         o.RK = mulk<3>(R1, k1);                    // Q60
         s = fx_mac(s, sg + (w >> 1), o.RK);        // Q61 x Q60
         o.s0 = fx_sum<1>(s);                       // Q58
-        o.E0 = mulk<6>(mulk<6>(tw, v2), S - (P >> 1)) + (fx_shl(mu, 2) >> n) - mulk<5>(bw, o.s0);
+        FxAcc e = fx_mul(mulk<5>(ntw, v2), (P >> 1) - S);  // 2 () in Q60 x Q60
+        e = fx_mac(e, nbw, o.s0);                          // Q62 x Q58; both doubled below
+        o.E0 = fx_sum<5>(e) + (fx_shl(mu, 2) >> n);
     }
     {
         FxAcc s = fx_mul(wt2, mulk<3>(dl, X0));            // Q62 x Q59
         s = fx_mac(s, mulk<3>(q.w, dl - sg), Y);           // 2 w~ (delta - sigma) in Q61 x Q60
         s = fx_mac(s, dl - fx_shl(sg, 1), Q);              // -(2 sigma - delta) Q61 x Q60
         o.s1 = fx_sum<1>(s);                               // Q58
-        FxAcc e = fx_mul(bw, -o.s1);                       // Q62 x Q58
-        e = fx_mac(e, isgk1, -wP);                         // Q60 x 2 w~ P in Q60
+        FxAcc e = fx_mul(nbw, o.s1);                       // Q62 x Q58
+        e = fx_mac(e, nigk1, wP);                          // Q60 x 2 w~ P in Q60
         e = fx_mac(e, t, mulk<6>(k1, v2));                 // Q60 x 2 K1 V2 in Q60
         e = fx_mac(e, dl, mu);                             // Q61 x Q59
         o.E1 = fx_sum<4>(e) - Q;
@@ -388,32 +391,33 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
         const fx F1 = fx_sum<1>(fx_mac(fx_mul(sg2 + wr2, k1), o.rww, k0));             // Q58
         const fx F2 = fx_sum<3>(fx_mac(fx_mul(dl, sg2), wr2, rho));                    // Q60
         const fx z = mulk<3>(mulk<2>(sc, isg3), q.ithp);                               // Q62
-        o.A = mulk<3>(a2w2, wt3) >> p;                              // 2 a^2 w^2 w~^3 2^-p in Q61
-        FxAcc e = fx_mul(o.A, mulk<1>(z, H));                       // x Q57
-        const fx g2 = mulk<2>(g.th2, mulk<3>(q.s2x, q.ithp));       // th''/th', Q58
-        e = fx_mac(e, (t >> 2) - g2, mulk<5>(k2, v2));              // Q58 x Q60
-        o.E2a = fx_sum<3>(e) - mulk<1>(isgk1, k2);                    // 2 () in Q57 is ()'s integer in Q58
+        o.A = mulk<3>(a2w2, wt3);                                   // 2 a^2 w^2 w~^3 2^-p in Q61
+        FxAcc e = fx_mul(o.A, mulk<1>(z, H));                       // x Q58
+        const fx g2 = mulk<3>(g.th2, mulk<3>(q.s2x, q.ithp));       // th''/th', Q59
+        e = fx_mac(e, (t >> 1) - g2, mulk<5>(k2, v2));              // Q59 x Q60
+        e = fx_mac(e, nigk1 >> 1, k2);                              // 2 () in Q58 x Q61
+        o.E2a = fx_sum<2>(e);
         o.F1 = F1; o.F2 = F2; o.z = z; o.g2 = g2;
         const fx G = mulk<3>(F2, v3) - (mulk<2>(aw, F1) >> u);      // Q57 (2 a w F1 in Q57)
         o.G = G;
         o.E2b = mulk<2>(fx_shl(z, q.ks), mulk<3>(k3, G));             // Q62 x Q57
     }
     {
-        o.B = mulk<2>(mulk<2>(g.a, bw), wt3) >> (p + u);                       // Q61
-        const FxAcc e = fx_mul(o.B, mulk<1>(k0, P) - H);                       // x -(H - 2 K0 P) Q58
-        o.E3a = fx_sum<2>(e) - mulk<1>(mulk<1>(gam, k3), k1 - (wP >> 1))         // Q60 x (2 K1 - w~ P) Q60
-              + (mulk<1>(awt >> p, M2) >> (u + 1))                             // a w kap2 th' K2/sigma: Q62 x Q59
-              - mulk<3>(tw, kv23);                                             // Q60 x Q60, times 4
-        const fx F3 = fx_sum<2>(fx_mac(fx_mul(ww, k0), sg2w, k1));             // Q60
-        const fx D = kv23 - (mulk<2>(mulk<2>(aw, isg2), mulk<3>(k2, F3)) >> u);  // Q60
-        o.E3b = mulk<3>(mulk<2>(mulk<2>(q.c, q.isn), q.thp), D);               // cot th' 2^-ks Q59 x Q60
+        o.B = mulk<2>(mulk<2>(g.a, nbw), wt3) >> u;                             // Q61
+        FxAcc e = fx_mul(o.B, H - mulk<2>(k0, P));                              // x (H - 2 K0 P) Q59
+        e = fx_mac(e, mulk<1>(gam, k3), (wP >> 1) - k1);                        // Q60 x (w~ P - 2 K1) Q60
+        e = fx_mac(e, ntw, kv23);                                               // 4 () in Q60 x Q60
+        o.E3a = fx_sum<1>(e) + (mulk<1>(awt >> p, M2) >> (u + 1));              // a w kap2 th' K2/sigma: Q62 x Q59
+        const fx F3 = fx_sum<2>(fx_mac(fx_mul(ww, k0), sg2w, k1));              // Q60
+        const fx D = (mulk<2>(mulk<2>(aw, isg2), mulk<3>(k2, F3)) >> u) - kv23;  // Q60
+        o.E3b = mulk<3>(mulk<2>(mulk<2>(q.c, q.isn), q.thp), D);                // -cot th' 2^-ks () Q59 x Q60
         o.F3 = F3;
         o.D = D;
     }
     // (terms that nothing reads cost nothing: the function is inlined)
     o.w = w; o.ww = ww; o.wt2 = wt2; o.wt3 = wt3; o.a2w2 = a2w2; o.s2 = s2; o.sg = sg; o.isg = isg;
-    o.rho = rho; o.dl = dl; o.isg2 = isg2; o.isg3 = isg3; o.beta = beta; o.bw = bw; o.gam = gam; o.aw = aw;
-    o.sc = sc; o.thi = thi; o.t = t; o.tw = tw; o.as2 = as2; o.P = P; o.R1 = R1; o.S = S; o.H = H; o.X0 = X0;
+    o.rho = rho; o.dl = dl; o.isg2 = isg2; o.isg3 = isg3; o.beta = beta; o.gam = gam; o.aw = aw;
+    o.sc = sc; o.thi = thi; o.t = t; o.as2 = as2; o.P = P; o.R1 = R1; o.S = S; o.H = H; o.X0 = X0;
     o.Y = Y; o.Q = Q; o.kap2 = kap2; o.kap3 = kap3; o.mu = mu; o.sg2 = sg2; o.wr2 = wr2;
 }
 
@@ -543,7 +547,7 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
             const fx hk = fx_shl(h, pt.ks);
             const fx p0 = mulk<3>(h, o.E0), p1 = mulk<3>(h, o.E1);  // Q61
             const fx p2 = mulk<6>(h, o.E2a) + (mulk<6>(hk, o.E2b) >> (2 * (pt.ks - s.u)));
-            const fx p3 = mulk<6>(h, o.E3a) - mulk<6>(hk, o.E3b);  // 2 E3b in Q57
+            const fx p3 = fx_sum<6>(fx_mac(fx_mul(h, o.E3a), hk, o.E3b));  // 2 E3b in Q57
             const int two = q == 1 ? 1 : 0;
             a1 += fx_shl(o1, two);
             a2 += fx_shl(o2, two);

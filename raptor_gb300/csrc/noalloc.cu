@@ -191,7 +191,7 @@ extern "C" int raptor_gpu_render_noalloc(int device, const double* d_cells, cons
     ls.block = kRayMaxBlock;
     ls.bps = occ > 0 ? occ : 1;
     ls.grid = sms * ls.bps;
-    ls.refill = kDefaultRefill;
+    ls.refill = fixed ? kDefaultRefillFast : kDefaultRefill;
     fn(ls, st, d_desc, n_imgs, 0, rays, d_ctr, d_I_out, TraceSpec{-1, nullptr, 0});
     if (cudaGetLastError() != cudaSuccess) return RAPTOR_ERR_CUDA;
     if (d_spectrum_out) {

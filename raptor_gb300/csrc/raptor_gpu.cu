@@ -545,7 +545,8 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
     return RAPTOR_OK;
 }
 
-LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form) {
+// fast: a fixed-point or double-float geodesic (kDefaultRefillFast)
+LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, bool fast) {
     LaunchShape ls;
     ls.block = ctx->opt.block_size > 0 ? ctx->opt.block_size : kRayMaxBlock;
     ls.block = std::max(32, std::min(kRayMaxBlock, ls.block / 32 * 32));
@@ -556,7 +557,7 @@ LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form) {
     ls.grid = ctx->num_sms * bps;
     ls.bps = bps;
     ls.refill = ctx->opt.refill_interval > 0 ? ctx->opt.refill_interval
-                                             : (form == RAPTOR_PREC_MIXED_DF ? kDefaultRefillDF : kDefaultRefill);
+                                             : (fast ? kDefaultRefillFast : kDefaultRefill);
     return ls;
 }
 
@@ -755,7 +756,7 @@ extern "C" int raptor_gpu_trace_ray(raptor_gpu_ctx* ctx, const raptor_image_desc
     CK(cudaMemsetAsync(ctx->d_trace, 0, bytes, ctx->stream));
     const void* fnp = nullptr;
     RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, false, false, 1);  // the trace kernels step in FP64
-    LaunchShape ls = default_shape(ctx, fnp, precision);
+    LaunchShape ls = default_shape(ctx, fnp, precision == RAPTOR_PREC_MIXED_DF);
     ls.grid = 1;
     ls.block = 32;
     TraceSpec tr{pixel, ctx->d_trace, max_records};

@@ -121,13 +121,13 @@ struct FxTangent {
         // the point
         const float r = Q(pt.r, 61), wt = Q(pt.w, 62), s = Q(pt.s, 62), c = Q(pt.c, 62), thp = Q(pt.thp, 60);
         const float ithp = Q(pt.ithp, 61), isn = fx_lead(pt.isn, exp2i(pt.ks - 29));
-        const float g2 = Q(o.g2, 58), th2 = g2 * thp;  // theta''/theta', theta''
+        const float g2 = Q(o.g2, 59), th2 = g2 * thp;  // theta''/theta', theta''
         const float dth = thp * dx2, ds = c * dth, dthp = th2 * dx2, dithp = -ithp * ithp * dthp;
         const float pt2 = ((thp - 3.14159274f) + 8.74227766e-8f) * dx2;
         const float dth2 = -(39.4784164f * pt2 + 1.16148634e-06f * pt2);  // -4 pi^2 (theta' - pi) dx2
         const float w = wt * pn, dw = -w * dx1, dwt = -wt * dx1;
         const float ww = w * wt, dww = -2.0f * ww * dx1, wt2 = Q(o.wt2, 62), dwt2 = -2.0f * wt2 * dx1;
-        const float wt3 = Q(o.wt3, 61), dwt3 = -3.0f * wt3 * dx1;
+        const float wt3 = wt2 * wt, dwt3 = -3.0f * wt3 * dx1;
         // metric functions
         const float aw = a * w + alo * w, daw = -aw * dx1;
         const float a2w2 = aw * aw, da2w2 = -2.0f * a2w2 * dx1;
@@ -145,7 +145,7 @@ struct FxTangent {
         // wave vector
         const float as2 = a * s2 + alo * s2, P = as2 * V3 * pu * pn, dP = (as2 * dV3 + a * ds2 * V3) * pu * pn;
         const float R1 = Q(o.R1, 60), dR1 = r * d1 + R1 * dx1, S = Q(o.S, 60), dS = d0 + dR1;
-        const float H = Q(o.H, 58), dH = 2.0f * S * dS;
+        const float H = Q(o.H, 59), dH = 2.0f * S * dS;
         const float X0 = Q(o.X0, 59), dX0 = 2.0f * ((k0 - P) * d0 - k0 * dP);
         const float Y = Q(o.Y, 60), dY = d1 * (k0 - P) + k1 * (d0 - dP);
         const float QQ = k1 * k1, dQ = 2.0f * k1 * d1;
@@ -196,7 +196,7 @@ struct FxTangent {
                           4.0f * (dtw * kv23 + tw * dkv23) - 2.0f * (dct * D + ct * dD);
         const float E0 = Q(o.E0, 60), E1 = Q(o.E1, 60);
         const float E2 = Q(o.E2a, 57) + Q(o.E2b, 57) * pu * pu * exp2i(-pt.ks);
-        const float E3 = Q(o.E3a, 57) - 2.0f * Q(o.E3b, 58) * exp2i(pt.ks);
+        const float E3 = Q(o.E3a, 57) + 2.0f * Q(o.E3b, 58) * exp2i(pt.ks);
 #undef Q
         const bool whole = q == end - 2 + (rk2 ? 1 : 0);
         const float h = whole ? L : 0.5f * L, dh = whole ? dL : 0.5f * dL;
