@@ -34,7 +34,8 @@
 //        - 4 t w K2 V3/sigma - 2 cot th' (K2 V3 - a w K2 (2 w w~ K0 + (sigma + 2w) K1)/sigma^2 2^-u)
 // Close to the axis sin theta = s~ 2^-ks is small, K3 and V3 2^u grow as its
 // reciprocal and L shrinks with it: the last terms of E2 and E3 are formed
-// without the factors 2^ks and applied with L 2^ks.
+// without the factors 2^ks and applied with L 2^ks; where that passes 1 (steps
+// along the axis with little angular momentum) the products are shifted after.
 //
 // A quantity "in Qf" is the integer value times 2^-f.  The ranges are those of
 // rays with n in [0, 13], p - n <= 3, x2 in [2^-13, 1 - 2^-13] and a step that
@@ -454,6 +455,13 @@ FX_HD void fx_normalise(FxState& s, fx lr) {
     }
 }
 
+// Bits by which L 2^ks is shortened to stay below 1: rays along the axis with
+// little angular momentum take steps that do not shrink with sin theta.
+FX_HD int fx_excess(int ks, fx L) {
+    const int e = ks + 2 - fx_clz((ufx)L);
+    return e > 0 ? e : 0;
+}
+
 // |d lambda| 2^(m-n) in Q62: L = eps m2 / (m2 (|K1| + |V3| 2^u) + |V2|), the
 // reciprocals of integrator.c:109-122 folded (its guards against zero rates
 // and steps do not act in this range).  False outside the ranges that the
@@ -469,9 +477,9 @@ FX_HD bool fx_step_size(const FxGeo& g, const FxState& s, int ks, fx& L) {
     const int kd = fx_clz((ufx)d) - 2;
     if (kd < 1 || kd > 20) return false;
     const fx y = mulk<1>(mulk<3>(g.eps, m2), fx_recip(fx_shl(d, kd)));  // Q65 x Q61: Q63; L = y 2^(kd-3)
-    if ((y >> (66 - kd - ks)) != 0) return false;                       // L 2^ks >= 1
+    if ((y >> (66 - kd)) != 0) return false;                            // L >= 1
     L = kd >= 4 ? fx_shl(y, kd - 4) : y >> (4 - kd);
-    return true;
+    return s.u == 0 || 2 * (ks - s.u) >= fx_excess(ks, L) + 2;
 }
 
 // One step of integrate_geodesic (integrator.c:109-146, 13-70) backward in
@@ -495,7 +503,8 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
     const fx full = -L, half = full >> 1;
     fx x1 = s.x1, x2 = s.x2, k0 = s.k0, k1 = s.k1, k2 = s.k2, k3 = s.k3;
     // RK4's sums start at the mean of what the floors of their products lose
-    fx a1 = 0, a2 = 4, b0 = 4, b1 = 4, b2 = 4, b3 = 4;
+    // (p2 has two of them)
+    fx a1 = 0, a2 = 4, b0 = 4, b1 = 4, b2 = 6, b3 = 4;
     const int end = rk2 ? 2 : 4;
 #ifdef __CUDACC__
 #pragma unroll 1
@@ -544,10 +553,11 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
             // is y + (o1 + 2 o2 + o3 + o4)/3; RK2: h f1, then y + d f2
             const fx h = q == end - 2 + (rk2 ? 1 : 0) ? full : half;
             const fx o1 = mulk<2>(h, k1), o2 = mulk<6>(h, v2);  // Q61, Q62
-            const fx hk = fx_shl(h, pt.ks);
+            const int ex = fx_excess(pt.ks, L);
+            const fx hk = fx_shl(h, pt.ks - ex);
             const fx p0 = mulk<3>(h, o.E0), p1 = mulk<3>(h, o.E1);  // Q61
-            const fx p2 = mulk<6>(h, o.E2a) + (mulk<6>(hk, o.E2b) >> (2 * (pt.ks - s.u)));
-            const fx p3 = fx_sum<6>(fx_mac(fx_mul(h, o.E3a), hk, o.E3b));  // 2 E3b in Q57
+            const fx p2 = mulk<6>(h, o.E2a) + (mulk<6>(hk, o.E2b) >> (2 * (pt.ks - s.u) - ex));
+            const fx p3 = fx_sum<6>(fx_mac(fx_mul(h, o.E3a), hk, fx_shl(o.E3b, ex)));  // 2 E3b in Q57
             const int two = q == 1 ? 1 : 0;
             a1 += fx_shl(o1, two);
             a2 += fx_shl(o2, two);

@@ -6,7 +6,9 @@
 // ray is where that arithmetic does not cover it: close to the polar axis,
 // with a very large angular wave vector, or not finite - the doubles x1, x2,
 // k^mu, which then step in FP64 (fx_slow_step) until they fit again.  On the
-// 1024x1024 image of the torus at 60 degrees that is 0.3 % of the steps.
+// 1024x1024 image of the torus at 60 degrees that is 0.02 % of the steps, at 2
+// degrees 0.3 % (30 % where L 2^ks was held below 1 instead of shortened,
+// fx_excess: FP64 771 ms against 298).
 #pragma once
 #include "ray_kernel.cuh"
 
