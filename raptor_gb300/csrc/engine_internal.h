@@ -98,7 +98,7 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
 // rays: how many the batch has
 RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed, long long rays);
 RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool, long long rays);
-RayLaunchFn pick_ray_kernel_df(int nf, const void** fn);
+RayLaunchFn pick_ray_kernel_df(int nf, const void** fn, long long rays);
 LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, bool fast);
 LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp);
 int enqueue_render(raptor_gpu_ctx* ctx, const Batch& b, int form, long long rb, long long re,

@@ -466,7 +466,7 @@ static void launch_ray_pool(const LaunchShape& ls, cudaStream_t st, const DevIma
 }
 
 RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed, long long rays) {
-    if (form == RAPTOR_PREC_MIXED_DF) return pick_ray_kernel_df(nf, fn);
+    if (form == RAPTOR_PREC_MIXED_DF) return pick_ray_kernel_df(nf, fn, rays);
     const bool mixed = form == RAPTOR_PREC_MIXED;
     if (fixed) return pick_ray_kernel_fx(nf, mixed, fn, pool, rays);
     // one instantiation per frequency-count bucket so tau/I stay in registers

@@ -182,14 +182,20 @@ __device__ __forceinline__ bool fx_in_grid(const DevImage& im, const FxState& c)
 
 // Blocks: 128-thread blocks per SM the kernels are compiled for.  They wait on
 // instruction fetch and on the multiply-adds' latency, which more warps hide,
-// but 4 blocks (128 registers) spill where 3 (168) hardly do.  FP64, one
-// frequency: 1024x1024 198 ms at 4 blocks, 205 at 3, 229 at 2; 800x800 122 and
-// 126; 512x512 59.1 and 57.3; 100x100 15.7 and 14.0: kFxManyRays rays and more
-// take 4.  The mixed kernels take 3 (1024x1024 127 ms either way, 512x512 41.4
-// and 39.3).  5 blocks (96 registers) are slower throughout.
+// but 4 blocks (128 registers) spill where 3 (168) hardly do and 2 (255) do
+// not at all; a launch of few rays per lane lasts as long as its longest rays
+// and is better off with fewer, quicker warps.  FP64, one frequency (ms at 4,
+// 3, 2 blocks): 1024x1024 195, 205, 229; 800x800 122, 126; 512x512 59.1, 52.6,
+// 58.7; 360x360 29.5 at 3, 31.1 at 2; 320x320 25.7, 25.1; 256x256 20.8, 19.4;
+// five frequencies 320x320 37.1, 38.4; 256x256 29.7, 27.6: kFxFewRays and
+// kFxManyRays rays part them.  Mixed (3, 2 blocks): 1024x1024 120 (127 at 4);
+// 512x512 33.9, 36.0; 400x400 22.9, 23.3; 360x360 20.5, 19.8; 256x256 16.7,
+// 14.8; 128x128 11.7, 10.7; five frequencies 320x320 24.0, 20.2: kFxFewRaysMixed.
+// 5 blocks (96 registers) are slower throughout.
 // A barrier per step (kLockstep) keeps the four warps of a pooled block on the
 // same code: 1024x1024 214 -> 202 ms.
-constexpr long long kFxManyRays = 1ll << 19;
+constexpr long long kFxFewRays = 3ll << 15, kFxManyRays = 1ll << 19;
+constexpr long long kFxFewRaysMixed = 1ll << 17;
 
 template <int NF, bool MIXED, int Blocks>
 struct FxRay {

@@ -223,13 +223,15 @@ __device__ __forceinline__ void finish_ray_df(const DevImage& im, const RayState
     if (kk == kk) c.kk_max = fmax(c.kk_max, kk);
 }
 
-// 3 blocks of 128 per SM: 168 registers a thread and no spills.  The DF
-// arithmetic wants warps to hide FP32 latency, but 4 blocks (128 registers,
-// a few hundred bytes of spills) were 2 % slower at 1024x1024, and 2 blocks
-// (8 warps at 196 registers) ran 1.4x slower.
-#ifndef RAPTOR_RAY_DF_MIN_BLOCKS
-#define RAPTOR_RAY_DF_MIN_BLOCKS 3
-#endif
+// Blocks: blocks of 128 per SM.  3 leave 168 registers a thread and no
+// spills; the DF arithmetic wants warps to hide FP32 latency, but 4 (128
+// registers, a few hundred bytes of spills) were 2 % slower at 1024x1024.  A
+// launch of few rays per lane lasts as long as its longest rays, and its fewer
+// warps run faster with 2 blocks' registers.  One frequency (ms at 3, 2
+// blocks): 1024x1024 67.0, 68.3; 512x512 18.8, 18.8; 450x450 15.0, 15.0;
+// 400x400 12.8, 12.2; 320x320 10.1, 8.7; 256x256 8.6, 7.7; 128x128 6.9, 5.5;
+// five frequencies 320x320 11.9, 10.2; 128x128 7.0, 6.6.
+constexpr long long kDfFewRays = 3ll << 16;
 
 // Each lane samples its own ray in place.  A sample pool as in the FP64
 // form (ray_kernel_pool: tickets of the sample's inputs in a per-warp
@@ -239,8 +241,8 @@ __device__ __forceinline__ void finish_ray_df(const DevImage& im, const RayState
 // this kernel's time, and the ring's bookkeeping and ticket traffic cost
 // more issue slots than the sample's half-empty warps waste.
 // TRACE: the per-step trace kernel (t and phi integrated, records written)
-template <int NF, bool TRACE>
-__global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_RAY_DF_MIN_BLOCKS)
+template <int NF, bool TRACE, int Blocks>
+__global__ void __launch_bounds__(kRayMaxBlock, Blocks)
     ray_kernel_df(const DevImage* __restrict__ imgs, int n_imgs, long long ray_begin, long long ray_end,
                   unsigned long long* __restrict__ counters, double* __restrict__ out, int refill_interval,
                   TraceSpec tr) {
@@ -298,11 +300,23 @@ __global__ void __launch_bounds__(kRayMaxBlock, RAPTOR_RAY_DF_MIN_BLOCKS)
 }
 
 // renders; a trace (any frequency count) takes the 8-frequency trace kernel
-template <int NF>
+template <int NF, int Blocks>
 void launch_ray_df(const LaunchShape& ls, cudaStream_t st, const DevImage* imgs, int n, long long b, long long e,
                    unsigned long long* ctr, double* out, TraceSpec tr) {
-    if (tr.out) ray_kernel_df<kMaxFreqs, true><<<ls.grid, ls.block, 0, st>>>(imgs, n, b, e, ctr, out, ls.refill, tr);
-    else ray_kernel_df<NF, false><<<ls.grid, ls.block, 0, st>>>(imgs, n, b, e, ctr, out, ls.refill, tr);
+    if (tr.out)
+        ray_kernel_df<kMaxFreqs, true, 3><<<ls.grid, ls.block, 0, st>>>(imgs, n, b, e, ctr, out, ls.refill, tr);
+    else
+        ray_kernel_df<NF, false, Blocks><<<ls.grid, ls.block, 0, st>>>(imgs, n, b, e, ctr, out, ls.refill, tr);
+}
+
+template <int NF, int Blocks>
+RayLaunchFn kernel_of(const void** fn) {
+    *fn = (const void*)ray_kernel_df<NF, false, Blocks>;
+    return launch_ray_df<NF, Blocks>;
+}
+template <int NF>
+RayLaunchFn pick(const void** fn, long long rays) {
+    return rays < kDfFewRays ? kernel_of<NF, 2>(fn) : kernel_of<NF, 3>(fn);
 }
 
 }  // namespace
@@ -310,10 +324,9 @@ void launch_ray_df(const LaunchShape& ls, cudaStream_t st, const DevImage* imgs,
 
 using namespace raptor;
 
-RayLaunchFn pick_ray_kernel_df(int nf, const void** fn) {
-    if (nf <= 1) { *fn = (const void*)ray_kernel_df<1, false>; return launch_ray_df<1>; }
-    if (nf <= 2) { *fn = (const void*)ray_kernel_df<2, false>; return launch_ray_df<2>; }
-    if (nf <= 4) { *fn = (const void*)ray_kernel_df<4, false>; return launch_ray_df<4>; }
-    *fn = (const void*)ray_kernel_df<8, false>;
-    return launch_ray_df<8>;
+RayLaunchFn pick_ray_kernel_df(int nf, const void** fn, long long rays) {
+    if (nf <= 1) return pick<1>(fn, rays);
+    if (nf <= 2) return pick<2>(fn, rays);
+    if (nf <= 4) return pick<4>(fn, rays);
+    return pick<8>(fn, rays);
 }
