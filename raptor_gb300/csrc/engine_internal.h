@@ -99,7 +99,9 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
 RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed, long long rays);
 RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool, long long rays);
 RayLaunchFn pick_ray_kernel_df(int nf, const void** fn, long long rays);
-LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, bool fast);
+// blocks per SM of a launch that names none
+int default_blocks(int form, bool fast, long long rays, int sms, int block, int occ);
+LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, long long rays);
 LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp);
 int enqueue_render(raptor_gpu_ctx* ctx, const Batch& b, int form, long long rb, long long re,
                    const LaunchShape& ls, RayLaunchFn fn, bool timed, raptor::TraceSpec tr = {-1, nullptr, 0});

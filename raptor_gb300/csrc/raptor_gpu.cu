@@ -545,15 +545,29 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
     return RAPTOR_OK;
 }
 
-// fast: a fixed-point or double-float geodesic (kDefaultRefillFast)
-LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, bool fast) {
+// As many as fit, but one where the whole launch is in flight at once: it then
+// lasts as long as its longest ray, which steps faster beside fewer warps.  For
+// the fixed-point and double-float geodesics, up to two rays per lane of such
+// a launch: mixed-DF 100x100 5.2 -> 4.4 ms, 190x191 6.1 -> 5.6; mixed 128x128
+// 11.5 -> 10.6, 190x191 12.8 -> 11.8; beyond, slower in some views (log-polar
+// 210x211 mixed 15.4 -> 17.1).  The FP64 form's samples keep more warps busy:
+// up to 3/2 (128x128 13.2 -> 12.5, 140x141 at three frequencies 17.2 -> 15.5;
+// 190x191 14.8 -> 15.6).
+int default_blocks(int form, bool fast, long long rays, int sms, int block, int occ) {
+    const long long lanes = (long long)sms * block;
+    return fast && rays * 2 <= lanes * (form == RAPTOR_PREC_FP64 ? 3 : 4) ? 1 : occ;
+}
+
+LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, long long rays) {
+    const bool fast = form == RAPTOR_PREC_MIXED_DF || fixed;
     LaunchShape ls;
     ls.block = ctx->opt.block_size > 0 ? ctx->opt.block_size : kRayMaxBlock;
     ls.block = std::max(32, std::min(kRayMaxBlock, ls.block / 32 * 32));
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, ls.block, 0);
     occ = std::max(occ, 1);
-    int bps = ctx->opt.blocks_per_sm > 0 ? std::min(ctx->opt.blocks_per_sm, occ) : occ;
+    int bps = ctx->opt.blocks_per_sm > 0 ? std::min(ctx->opt.blocks_per_sm, occ)
+                                         : default_blocks(form, fast, rays, ctx->num_sms, ls.block, occ);
     ls.grid = ctx->num_sms * bps;
     ls.bps = bps;
     ls.refill = ctx->opt.refill_interval > 0 ? ctx->opt.refill_interval
@@ -756,7 +770,7 @@ extern "C" int raptor_gpu_trace_ray(raptor_gpu_ctx* ctx, const raptor_image_desc
     CK(cudaMemsetAsync(ctx->d_trace, 0, bytes, ctx->stream));
     const void* fnp = nullptr;
     RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, false, false, 1);  // the trace kernels step in FP64
-    LaunchShape ls = default_shape(ctx, fnp, precision == RAPTOR_PREC_MIXED_DF);
+    LaunchShape ls = default_shape(ctx, fnp, precision, false, 1);
     ls.grid = 1;
     ls.block = 32;
     TraceSpec tr{pixel, ctx->d_trace, max_records};

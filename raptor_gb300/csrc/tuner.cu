@@ -66,7 +66,7 @@ void save_file_cache(const std::string& key, const LaunchShape& ls) {
 }  // namespace
 
 LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp) {
-    LaunchShape base = default_shape(ctx, fnp, form == RAPTOR_PREC_MIXED_DF || b.fixed);
+    LaunchShape base = default_shape(ctx, fnp, form, b.fixed, b.total_rays);
     if (!ctx->opt.autotune) return base;
     load_file_cache(ctx);
     const std::string key = signature(ctx, b, form);
@@ -98,6 +98,7 @@ LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunc
             cands.push_back(ls);
         }
     }
+    if (base.bps == 1) cands.push_back(base);  // a launch of all its rays at once (default_blocks)
     const long long lanes = (long long)ctx->num_sms * 3 * 128;
     const long long n = std::min<long long>(b.total_rays, 6 * lanes);
     const long long rb = (b.total_rays - n) / 2, re = rb + n;

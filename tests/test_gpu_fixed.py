@@ -105,3 +105,22 @@ def test_mixed_adjoint_matches_fp64(eng, case):
     for key in ("d_m_unit", "d_r_high", "d_r_low", "d_inclination"):
         scale = max(abs(g[key]), 1e-6 * abs(g["d_r_high"]))
         assert abs(m[key] - g[key]) <= 2e-3 * scale, (key, m[key], g[key])
+
+
+@pytest.mark.parametrize("prec,inside,outside", [(0, (170, 171), (171, 171)), (1, (197, 197), (198, 197)),
+                                                 (2, (197, 197), (198, 197))], ids=["fp64", "mixed", "mixed_df"])
+def test_small_launches_take_one_block_per_sm(eng, torus64, prec, inside, outside):
+    """At both sides of the line the launch's shape changes no bit."""
+    from raptor_gb300 import engine
+    ref = engine.Engine(blocks_per_sm=2)
+    ga, gb = (e.upload_grid(torus64.geom, torus64.prims) for e in (eng, ref))
+    lanes = 0
+    for size, blocks in ((inside, 1), (outside, 2)):
+        a, _ = eng.render(engine.image_desc(*size, [230e9], grid=ga, stepsize=0.1), prec)
+        st = eng.stats()
+        lanes = st["grid_blocks"] // st["blocks_per_sm"] * st["block_size"]
+        if lanes == 152 * 128:
+            assert st["blocks_per_sm"] == blocks
+        b, _ = ref.render(engine.image_desc(*size, [230e9], grid=gb, stepsize=0.1), prec)
+        assert np.array_equal(a, b) and np.any(a)
+    ref.close()
