@@ -1008,7 +1008,15 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
                 ? (b.fixed ? pick_vjp_fx : pick_vjp_mixed)(b.max_nf, &kp, kappa, one_pass)
                 : pick_vjp_fp64(b.max_nf, &kp, !ctx->opt.no_sample_pool, &scratch_rows, kappa, one_pass);
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kp, kVjpBlock, 0));
-        const int grid = ctx->num_sms * std::max(occ, 1);
+        // The pooled FP64 adjoint takes one block per SM up to five rays per lane
+        // of such a launch: the queue then deals the rays evenly, where eight
+        // warps per SM leave some SMs twice the others' share of the FP64 pipe's
+        // work, and four keep that pipe as busy.  128x128 83 -> 65 ms (and 15 %
+        // from run to run -> 1 %), 256x255 126 -> 107, 300x301 152 -> 141;
+        // 340x341 and above within 2 % either way.
+        const bool even = precision == RAPTOR_PREC_FP64 && !ctx->opt.no_sample_pool &&
+                          re - rb <= 5ll * ctx->num_sms * kVjpBlock;
+        const int grid = ctx->num_sms * (even ? 1 : std::max(occ, 1));
         // the pooled adjoint's per-warp result slices (several frequencies)
         if (scratch_rows > 0) {
             rc = ensure_buffer(ctx, (void**)&ctx->d_vjp_scratch, &ctx->vjp_scratch_cap,

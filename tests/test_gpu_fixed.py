@@ -124,3 +124,22 @@ def test_small_launches_take_one_block_per_sm(eng, torus64, prec, inside, outsid
         b, _ = ref.render(engine.image_desc(*size, [230e9], grid=gb, stepsize=0.1), prec)
         assert np.array_equal(a, b) and np.any(a)
     ref.close()
+
+
+def test_fp64_adjoint_grids_agree(eng, torus64):
+    """312x312 rays are more than five per lane of one block per SM, its halves
+    fewer: the image's gradients are the halves' sums, to the order of the
+    FP64 sums (1e-12)."""
+    from raptor_gb300 import engine
+    gid = eng.upload_grid(torus64.geom, torus64.prims)
+    desc = engine.image_desc(312, 312, [230e9], grid=gid, inclination=60.0, stepsize=0.1)
+    w = np.ones(312 * 312)
+    _, g = eng.vjp(desc, w, engine.PREC_FP64, want_fields=False)
+    whole = eng.stats()["grid_blocks"]
+    half = 312 * 156
+    _, lo = eng.vjp(desc, w, engine.PREC_FP64, want_fields=False, ray_begin=0, ray_count=half)
+    assert eng.stats()["grid_blocks"] * 2 == whole or whole != 2 * 152
+    _, hi = eng.vjp(desc, w, engine.PREC_FP64, want_fields=False, ray_begin=half, ray_count=half)
+    for key in ("d_m_unit", "d_r_high", "d_r_low", "d_inclination"):
+        parts = abs(lo[key]) + abs(hi[key])
+        assert abs(lo[key] + hi[key] - g[key]) <= 1e-12 * parts, key
