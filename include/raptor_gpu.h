@@ -51,8 +51,10 @@ extern "C" {
                                  stats count them in n_stepcap.  Text in last_error. */
 
 /* arithmetic forms */
-#define RAPTOR_PREC_FP64 0  /* everything FP64, the reference's arithmetic */
-#define RAPTOR_PREC_MIXED 1 /* FP64 geodesic + metric, FP32 fluid/emission/transfer */
+#define RAPTOR_PREC_FP64 0  /* FP64 transfer, the geodesic at least as precise: 64-bit fixed point
+                               (56 to 61 fraction bits) where R0 = 0, 0.2 <= hslope <= 1.8 and
+                               1e-7 <= stepsize <= 0.1 for every image of the call, else FP64 */
+#define RAPTOR_PREC_MIXED 1 /* geodesic as RAPTOR_PREC_FP64, FP32 fluid/emission/transfer */
 #define RAPTOR_PREC_MIXED_DF 2 /* geodesic + metric in double-float (pairs of FP32, 48-bit
                                   significand) on the FP32 pipes, transfer as RAPTOR_PREC_MIXED */
 
@@ -218,14 +220,15 @@ int raptor_gpu_trace_ray(raptor_gpu_ctx *ctx, const raptor_image_desc *img, int 
  * layout and nu^3 scaling as I_out), returns dL/d(M_UNIT, R_HIGH, R_LOW,
  * INCLINATION) and, if the pointers are set, the per-cell gradients on the
  * image's grid.  precision selects the form and its adjoint pass (FP64:
- * FP64 tangents and dual sample; mixed: the FP64 geodesic with FP32 tangents
- * and the FP32 dual sample; mixed-DF: the double-float geodesic with FP32
+ * FP64 geodesic, tangents and dual sample; mixed: the form's geodesic with
+ * FP32 tangents and the FP32 dual sample; mixed-DF: the double-float geodesic with FP32
  * tangents and sample).  By default the adjoint runs in one pass, taking
  * each ray's I from its own sums and keeping the ray's per-cell terms on a
  * device tape until the ray ends (raptor_gpu_options.vjp_tape); I_out
  * (may be NULL) then receives the image that pass renders, equal to
- * raptor_gpu_render's to rounding (1e-11 of the largest pixel in FP64, 1e-5
- * with the FP32 transfers).  In two passes (vjp_tape = -1, the in-place FP64
+ * raptor_gpu_render's to rounding (in FP64, whose adjoint steps the geodesic
+ * in FP64, 1e-11 of the largest pixel but for rays that circle the hole, which
+ * amplify it to 1e-9; 1e-5 with the FP32 transfers).  In two passes (vjp_tape = -1, the in-place FP64
  * adjoint, or a tape too small) the form's forward render runs first and
  * I_out receives it.
  * No counterpart in the reference, which has no derivatives. */
