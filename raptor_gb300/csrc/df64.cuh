@@ -69,6 +69,29 @@ __device__ __forceinline__ DF add_f(DF a, float b) {
     return DF{s.hi, __fadd_rn(s.lo, a.lo)};
 }
 __device__ __forceinline__ DF operator-(DF a, DF b) { return a + (-b); }
+// The same sums where |a| >= |b|: Dekker's fast two-sum has the same exact
+// error in 3 operations instead of 6.  (Were the order broken, it would be off
+// by an ulp of the lo part's scale.)  1024x1024 69.1 -> 68.2 ms, its
+// 512x512 five-frequency VJP 52.5 -> 51.6, with the scaled sums below.
+__device__ __forceinline__ DF add_ordered(DF a, DF b) {
+    const DF s = quick_two_sum(a.hi, b.hi);
+    return DF{s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo))};
+}
+__device__ __forceinline__ DF add_ordered(DF a, float b) {
+    const DF s = quick_two_sum(a.hi, b);
+    return DF{s.hi, __fadd_rn(s.lo, a.lo)};
+}
+__device__ __forceinline__ DF add_ordered(float a, DF b) {
+    const DF s = quick_two_sum(a, b.hi);
+    return DF{s.hi, __fadd_rn(s.lo, b.lo)};
+}
+// a + w b for a power of two w: its products are exact, so they fold into the sums
+__device__ __forceinline__ DF add_scaled(DF a, DF b, float w) {
+    const float s = __fmaf_rn(b.hi, w, a.hi);
+    const float bb = __fsub_rn(s, a.hi);
+    const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fmaf_rn(b.hi, w, -bb));
+    return DF{s, __fadd_rn(e, __fmaf_rn(b.lo, w, a.lo))};
+}
 
 // |lo| <= ulp(hi)/2 again
 __device__ __forceinline__ DF df_norm(DF a) { return quick_two_sum(a.hi, a.lo); }
@@ -137,6 +160,12 @@ __device__ __forceinline__ DF operator/(DF a, double c) { return a / df_const(c)
 
 __device__ __forceinline__ DF fma(DF a, DF b, DF c) { return a * b + c; }
 __device__ __forceinline__ DF fma(DF a, DF b, double c) { return a * b + c; }
+__device__ __forceinline__ DF fma_large(DF a, DF b, DF c) { return add_ordered(a * b, c); }
+__device__ __forceinline__ DF fma_small(DF a, DF b, DF c) { return add_ordered(c, a * b); }
+__device__ __forceinline__ DF fma_small(DF a, DF b, double c) {
+    const DF k = df_const(c);
+    return k.lo == 0.0f ? add_ordered(k.hi, a * b) : add_ordered(k, a * b);
+}
 
 // ----------------------------------------------------------- comparisons
 // by the sign of the difference rounded to FP32
@@ -169,10 +198,10 @@ __device__ __forceinline__ DF fast_exp(DF x) {
     t = __fmaf_rn(t, q, 1.0f / 6.0f);
     t = __fmul_rn(__fmul_rn(t, q), __fmul_rn(q, q));
     const DF r2 = r * r;
-    const DF em1 = add_f(r + DF{__fmul_rn(r2.hi, 0.5f), __fmul_rn(r2.lo, 0.5f)}, t);
+    const DF em1 = add_ordered(add_ordered(r, DF{__fmul_rn(r2.hi, 0.5f), __fmul_rn(r2.lo, 0.5f)}), t);
     const float2 T2 = __ldg(&kExp2TableDF[m & 63]);
     const DF T{T2.x, T2.y};
-    const DF v = T + T * em1;
+    const DF v = add_ordered(T, T * em1);
     const float sc = __int_as_float(((m >> 6) + 127) << 23);  // 2^(m/64 integer part)
     return DF{__fmul_rn(v.hi, sc), __fmul_rn(v.lo, sc)};
 }
@@ -190,10 +219,10 @@ __device__ __forceinline__ void fast_sincospi(DF x, DF* s, DF* c) {
     const float a2f = a2.hi;
     const float a4 = __fmul_rn(a2f, a2f);
     const float srest = __fmul_rn(a4, __fmaf_rn(a2f, 1.0f / 5040.0f, -1.0f / 120.0f));
-    const DF q = add_f(a2 * DF{kSixthDFhi, kSixthDFlo}, srest);  // a^2/6 - a^4/120 + a^6/5040
-    const DF sa = a - a * q;
+    const DF q = add_ordered(a2 * DF{kSixthDFhi, kSixthDFlo}, srest);  // a^2/6 - a^4/120 + a^6/5040
+    const DF sa = add_ordered(a, -(a * q));
     const float crest = __fmul_rn(a4, __fmaf_rn(a2f, -1.0f / 720.0f, 1.0f / 24.0f));
-    const DF cm1 = add_f(DF{__fmul_rn(a2.hi, -0.5f), __fmul_rn(a2.lo, -0.5f)}, crest);
+    const DF cm1 = add_ordered(DF{__fmul_rn(a2.hi, -0.5f), __fmul_rn(a2.lo, -0.5f)}, crest);
     const float4 T = __ldg(&kSinCosPiTableDF[n & 255]);
     const DF S{T.x, T.y}, C{T.z, T.w};
     *s = add_norm(S, S * cm1 + C * sa);

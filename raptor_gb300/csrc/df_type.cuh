@@ -45,6 +45,22 @@ struct GeoDF {
     DF one_m_h, th_coef;
 };
 
+// a + b with |a| >= |b|, a b + c with |a b| >= |c| (fma_large) or |a b| <= |c|
+// (fma_small), a + w b with w a power of two: the plain operations, for which
+// double-float values (df64.cuh) have shorter forms with the same result.
+template <class A, class B>
+__host__ __device__ __forceinline__ auto add_ordered(const A& a, const B& b) {
+    return a + b;
+}
+template <class A, class B, class C>
+__device__ __forceinline__ auto fma_large(const A& a, const B& b, const C& c) {
+    return fma(a, b, c);
+}
+template <class A, class B, class C>
+__device__ __forceinline__ auto fma_small(const A& a, const B& b, const C& c) {
+    return fma(a, b, c);
+}
+
 // Type of the RK stage weights for a state type: FP64 constants for double
 // and dual numbers, FP32 for DF (df64.cuh).
 template <class R>

@@ -195,6 +195,36 @@ __host__ __device__ inline Dual<N, T, TD> operator*(const Dual<N, T, TD>& a, flo
     return r;
 }
 
+// the ordered sums of double-float values (df64.cuh)
+template <int N, class T, class TD, if_not_double<T> = 0>
+__device__ inline Dual<N, T, TD> add_ordered(const Dual<N, T, TD>& a, const Dual<N, T, TD>& b) {
+    Dual<N, T, TD> r;
+    r.v = add_ordered(a.v, b.v);
+#pragma unroll
+    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] + b.d[i];
+    return r;
+}
+template <int N, class T, class TD, if_not_double<T> = 0>
+__device__ inline Dual<N, T, TD> add_ordered(const Dual<N, T, TD>& a, const T& b) {
+    Dual<N, T, TD> r = a;
+    r.v = add_ordered(a.v, b);
+    return r;
+}
+template <int N, class T, class TD, if_not_double<T> = 0>
+__device__ inline Dual<N, T, TD> fma_large(const Dual<N, T, TD>& a, const Dual<N, T, TD>& b, const Dual<N, T, TD>& c) {
+    return add_ordered(a * b, c);
+}
+template <int N, class T, class TD, if_not_double<T> = 0>
+__device__ inline Dual<N, T, TD> fma_small(const T& a, const Dual<N, T, TD>& b, const Dual<N, T, TD>& c) {
+    return add_ordered(c, a * b);
+}
+template <int N, class T, class TD, if_not_double<T> = 0>
+__device__ inline Dual<N, T, TD> fma_small(const T& a, const Dual<N, T, TD>& b, double c) {
+    Dual<N, T, TD> r = a * b;
+    r.v = add_ordered(scalar_cast<T>(c), r.v);
+    return r;
+}
+
 template <int N, class T, class TD> __host__ __device__ inline Dual<N, T, TD>& operator+=(Dual<N, T, TD>& a, const Dual<N, T, TD>& b) { a = a + b; return a; }
 template <int N, class T, class TD> __host__ __device__ inline Dual<N, T, TD>& operator-=(Dual<N, T, TD>& a, const Dual<N, T, TD>& b) { a = a - b; return a; }
 template <int N, class T, class TD> __host__ __device__ inline Dual<N, T, TD>& operator*=(Dual<N, T, TD>& a, const Dual<N, T, TD>& b) { a = a * b; return a; }

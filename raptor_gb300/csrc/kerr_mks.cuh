@@ -73,9 +73,9 @@ __device__ __forceinline__ void mks_point(R x1, R x2, const G& g, MksPointT<R>& 
     p.r = g.R0 + p.rp;
     fast_sincospi(2.0 * x2, &p.s2x, &p.c2x);
     // theta = pi x2 + (1-h)/2 sin(2 pi x2) (metric.c:98), evaluated as sinpi/cospi of theta/pi
-    fast_sincospi(fma(g.th_coef, p.s2x, x2), &p.s, &p.c);
-    const R Sg = fma(p.r, p.r, g.a2 * p.c * p.c);
-    const R thp = CUDART_PI * fma(g.one_m_h, p.c2x, 1.0);
+    fast_sincospi(fma_small(g.th_coef, p.s2x, x2), &p.s, &p.c);
+    const R Sg = fma_large(p.r, p.r, g.a2 * p.c * p.c);
+    const R thp = CUDART_PI * fma_small(g.one_m_h, p.c2x, 1.0);
     point_reciprocals(Sg, thp, p);
 }
 
@@ -94,12 +94,12 @@ __device__ __forceinline__ void mks_point_rolled(R x1, R x2, const G& g, MksPoin
         p.s2x = sv;
         p.c2x = cv;
         // theta = pi x2 + (1-h)/2 sin(2 pi x2) (metric.c:98), as theta / pi
-        arg = fma(g.th_coef, sv, x2);
+        arg = fma_small(g.th_coef, sv, x2);
     }
     p.s = sv;
     p.c = cv;
-    const R Sg = fma(p.r, p.r, g.a2 * p.c * p.c);
-    const R thp = CUDART_PI * fma(g.one_m_h, p.c2x, 1.0);
+    const R Sg = fma_large(p.r, p.r, g.a2 * p.c * p.c);
+    const R thp = CUDART_PI * fma_small(g.one_m_h, p.c2x, 1.0);
     point_reciprocals(Sg, thp, p);
 }
 
@@ -119,12 +119,12 @@ __device__ __forceinline__ void geodesic_accel(const MksPointT<R>& p, const G& g
     const R s2th = 2.0 * sc;
     const R cot = c * p.isn;
     const R Sg = p.Sg, Sg2 = Sg * Sg;
-    const R r2a2 = r2 + a2;
+    const R r2a2 = add_ordered(r2, a2);  // r > 1 >= a outside the horizon
     const R two_r = 2.0 * r;
-    const R Dl = r2a2 - two_r;
+    const R Dl = add_ordered(r2a2, -two_r);  // Delta > 0
     const R Rr2 = two_r * r2a2;  // 2 r (r^2 + a^2)
     const R iS = p.iS, iS2 = iS * iS, iS3 = iS2 * iS;
-    const R B = (2.0 * r2 - Sg) * iS3;
+    const R B = add_ordered(2.0 * r2, -Sg) * iS3;
     const R riS = r * iS;
     const R as2 = a * s2;
     const R aB = a * B;

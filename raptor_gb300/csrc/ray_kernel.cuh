@@ -220,6 +220,10 @@ template <class R, class W>
 __device__ __forceinline__ R stage_scale(const R& f, W w) {
     return f * w;
 }
+template <class R, class W>
+__device__ __forceinline__ R add_scaled(const R& a, const R& f, W w) {
+    return a + stage_scale(f, w);
+}
 
 // The same RK4 step with all four stages and the end point's evaluation in
 // one rolled loop, so the stage body (point transcendentals, connection,
@@ -246,7 +250,7 @@ __device__ __forceinline__ void rk4_step_rolled(const G& g, R y[8], MksPointT<R>
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 if (!rk_updates<TPhi>(i)) continue;
-                acc[i] = (q == 0) ? f[i] : acc[i] + stage_scale(f[i], wacc);
+                acc[i] = (q == 0) ? f[i] : add_scaled(acc[i], f[i], wacc);
                 ys[i] = y[i] + dnext * f[i];
             }
         } else {
