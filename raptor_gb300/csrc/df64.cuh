@@ -168,8 +168,12 @@ __device__ __forceinline__ DF fma_small(DF a, DF b, double c) {
 }
 
 // ----------------------------------------------------------- comparisons
-// by the sign of the difference rounded to FP32
-__device__ __forceinline__ bool operator<(DF a, DF b) { return df_value(a - b) < 0.0f; }
+// by the sign of the difference rounded to FP32: where the leading parts are
+// within a factor of two of each other their difference is exact, elsewhere
+// it decides alone
+__device__ __forceinline__ bool operator<(DF a, DF b) {
+    return __fadd_rn(__fsub_rn(a.hi, b.hi), __fsub_rn(a.lo, b.lo)) < 0.0f;
+}
 __device__ __forceinline__ bool operator>(DF a, DF b) { return b < a; }
 __device__ __forceinline__ bool operator<=(DF a, DF b) { return !(b < a); }
 __device__ __forceinline__ bool operator>=(DF a, DF b) { return !(a < b); }
