@@ -17,7 +17,7 @@
 // V2, V3 = K2, K3 2^(p-n) (= 2^n k^2, 2^(n-u) k^3) and L = d lambda 2^(m-n), so that
 //   x1' = K1, x2' = V2 and K' = E per unit of L.
 // The Kerr-Schild connection (metric.c:538-638) in these units has no factor
-// larger than a few: with w = 1/r, sigma = Sigma w^2, delta = Delta w^2,
+// larger than 8/th' <= 13 (the axis term of E2 at hslope 1.8): with w = 1/r, sigma = Sigma w^2, delta = Delta w^2,
 // rho = 1 + a^2 w^2, s = sin theta, c = cos theta, th' = d theta/d x2,
 //   beta = (2 - sigma)/sigma^3 (Christoffel's B r^4), gamma = 1/sigma - a^2 s^2 beta w^3 (C r),
 //   P = a s^2 k^3, t = a^2 s c th' w^2/sigma, kap2 = th' V2, kap3 = s V3 2^u,
@@ -57,6 +57,12 @@ struct longlong2 {
 #define FX_HD static inline
 #define FX_MEMBER inline
 #define FX_TABLE(name, n) static const longlong2 name[n]
+#endif
+
+// FX_KEPT(ok): ok holds where an operation keeps every bit of its value.  The
+// CPU range check (tests/fixed_kept.h) defines it; nothing is tested here.
+#ifndef FX_KEPT
+#define FX_KEPT(ok)
 #endif
 
 namespace raptor {
@@ -155,13 +161,18 @@ FX_HD FxAcc fx_mac(FxAcc r, fx a, fx b) {
     r.h = fx_wide(ah, bh, r.h);
     return r;
 }
+FX_HD bool fx_fits(fx a, int s) { return s < 64 && (fx)((ufx)a << s) >> s == a; }
 // Value of the sum times 2^(K - 64), 1 <= K < 32.  (K = 0, which would leave
 // the low half of c unused, is avoided throughout: the compiler then takes
 // the multiply-add's high-half form, at less than half the rate.)
+FX_HD fx fx_sum(FxAcc r, int K) {
+    const fx h = fx_add32((int)fx_u1(r.c), r.h);
+    FX_KEPT(fx_fits(h, K));
+    return fx_pair(fx_funnel(fx_u0(r.c), fx_u0(h), K), fx_funnel(fx_u0(h), fx_u1(h), K));
+}
 template <int K>
 FX_HD fx fx_sum(FxAcc r) {
-    const fx h = fx_add32((int)fx_u1(r.c), r.h);
-    return fx_pair(fx_funnel(fx_u0(r.c), fx_u0(h), K), fx_funnel(fx_u0(h), fx_u1(h), K));
+    return fx_sum(r, K);
 }
 // a b 2^(K - 64): factors in Qx and Qy give Q(x + y - 64 + K)
 template <int K>
@@ -174,9 +185,13 @@ FX_HD fx sqrk(fx a) {
     const int ah = fx_hi(a), al = fx_lo(a);
     const fx c = fx_wide(ah, al);
     const fx h = fx_add32((int)fx_funnel(fx_u0(c), fx_u1(c), 1), fx_wide(ah, ah));
+    FX_KEPT(fx_fits(h, K));
     return fx_pair(fx_funnel(fx_u0(c) << 1, fx_u0(h), K), fx_funnel(fx_u0(h), fx_u1(h), K));
 }
-FX_HD fx fx_shl(fx a, int s) { return (fx)((ufx)a << s); }
+FX_HD fx fx_shl(fx a, int s) {
+    FX_KEPT(fx_fits(a, s));
+    return (fx)((ufx)a << s);
+}
 // a 2^s for either sign of s, |s| < 64
 FX_HD fx fx_scale(fx a, int s) { return s >= 0 ? fx_shl(a, s) : a >> -s; }
 FX_HD fx fx_abs(fx a) { return a < 0 ? -a : a; }
@@ -556,7 +571,10 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
             const int ex = fx_excess(pt.ks, L);
             const fx hk = fx_shl(h, pt.ks - ex);
             const fx p0 = mulk<3>(h, o.E0), p1 = mulk<3>(h, o.E1);  // Q61
-            const fx p2 = mulk<6>(h, o.E2a) + (mulk<6>(hk, o.E2b) >> (2 * (pt.ks - s.u) - ex));
+            // hk E2b reaches 8/th' along the axis (13 at hslope 1.8): two bits
+            // of the shift are left out of the product, where there are two
+            const int sh = 2 * (pt.ks - s.u) - ex, up = sh >= 2 ? 2 : 0;
+            const fx p2 = mulk<6>(h, o.E2a) + (fx_sum(fx_mul(hk, o.E2b), 6 - up) >> (sh - up));
             const fx p3 = fx_sum<6>(fx_mac(fx_mul(h, o.E3a), hk, fx_shl(o.E3b, ex)));  // 2 E3b in Q57
             const int two = q == 1 ? 1 : 0;
             a1 += fx_shl(o1, two);

@@ -1,0 +1,33 @@
+"""The number ranges of the fixed-point geodesic (csrc/fixed_geodesic.cuh) on
+the CPU: a build in which every product, shift and sum that loses bits of its
+value ends the program, over both ends of the grids' range and views from the
+polar axis to the equator.  A product that wraps is off by its format's range,
+and the ray by 1e-4 or far more: its final state is held to 1e-7 of long
+double."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+TESTS = os.path.join(ROOT, "tests")
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("kept") / "fixed_check")
+    subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fsanitize=signed-integer-overflow",
+                    "-fsanitize-undefined-trap-on-error", "-include", os.path.join(TESTS, "fixed_kept.h"),
+                    "-x", "c++", "-o", exe, os.path.join(TESTS, "fixed_check.cpp"), "-lm"], check=True)
+    return exe
+
+
+@pytest.mark.parametrize("inclination", [1.0, 2.0, 5.0, 10.0, 17.0, 30.0, 90.0, 160.0, 179.0])
+@pytest.mark.parametrize("hslope", [0.2, 1.0, 1.4, 1.8])
+def test_no_bits_are_lost(check, hslope, inclination):
+    for eps, integ, spin in ((0.05, 4, 0.9375), (0.1, 2, -0.998)):
+        run = subprocess.run([check, "500", str(eps), str(integ), str(spin), str(hslope), str(inclination), "40", "3"],
+                             capture_output=True, text=True)
+        assert run.returncode == 0, "an operation lost bits of its value"
+        worst = float(run.stdout.split()[13])
+        assert worst <= 1e-7, worst
