@@ -485,14 +485,14 @@ FX_HD bool fx_step_size(const FxGeo& g, const FxState& s, int ks, fx& L) {
     const int e = s.p - s.n;
     const fx m2 = fx_min(s.x2, fx_one(62) - s.x2);
     if (s.raw || s.n < 0 || s.n > 13 || e > 3 || s.u > 11 || (s.u > 0 && s.u >= ks) || m2 < fx_one(49)) return false;
-    const fx m2u = fx_shl(m2, s.u);
     if (((m2 >> 1) >> (61 - s.u)) != 0) return false;
+    const fx m2u = fx_shl(m2, s.u);
     const fx v2 = fx_abs(fx_vshift(s.k2, e)), v3 = fx_abs(fx_vshift(s.k3, e));
     const fx d = fx_sum<3>(fx_mac(fx_mul(m2, fx_abs(s.k1) >> 3), m2u, v3)) + (v2 << 1);  // Q59
     const int kd = fx_clz((ufx)d) - 2;
     if (kd < 1 || kd > 20) return false;
     const fx y = mulk<1>(mulk<3>(g.eps, m2), fx_recip(fx_shl(d, kd)));  // Q65 x Q61: Q63; L = y 2^(kd-3)
-    if ((y >> (66 - kd)) != 0) return false;                            // L >= 1
+    if (kd > 2 && (y >> (66 - kd)) != 0) return false;                  // L >= 1 (below kd = 3 it cannot be)
     L = kd >= 4 ? fx_shl(y, kd - 4) : y >> (4 - kd);
     return s.u == 0 || 2 * (ks - s.u) >= fx_excess(ks, L) + 2;
 }
