@@ -59,10 +59,12 @@ struct longlong2 {
 #define FX_TABLE(name, n) static const longlong2 name[n]
 #endif
 
-// FX_KEPT(ok): ok holds where an operation keeps every bit of its value.  The
-// CPU range check (tests/fixed_kept.h) defines it; nothing is tested here.
+// FX_KEPT(ok): ok holds where an operation keeps every bit of its value;
+// FX_TRACK(code) is what it takes to know.  The CPU range check
+// (tests/fixed_kept.h) defines them; nothing is tested here.
 #ifndef FX_KEPT
 #define FX_KEPT(ok)
+#define FX_TRACK(code)
 #endif
 
 namespace raptor {
@@ -147,18 +149,31 @@ FX_HD int fx_lo(fx a) { return (int)(unsigned)a; }
 // out: within 1/4 of 2^64 per product, which is 2^-60 for factors in Q62.
 struct FxAcc {
     fx h, c;
+    FX_TRACK(double most;)  // of |c|, whatever the low halves
 };
 FX_HD FxAcc fx_mul(fx a, fx b) {
     const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
     FxAcc r;
     r.c = fx_wide(al, bh, fx_wide(ah, bl));
     r.h = fx_wide(ah, bh);
+    FX_TRACK(r.most = fx_most(ah, bh);)
     return r;
 }
 FX_HD FxAcc fx_mac(FxAcc r, fx a, fx b) {
     const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
     r.c = fx_wide(al, bh, fx_wide(ah, bl, r.c));
     r.h = fx_wide(ah, bh, r.h);
+    FX_TRACK(r.most += fx_most(ah, bh);)
+    FX_KEPT(r.most < 0x1p63);
+    return r;
+}
+// The same sum with c's upper half moved into h.  A product adds as much as
+// half of |a| + |b| to |c|: sums whose factors' magnitudes come to 2^64 or
+// more take this on the way.
+FX_HD FxAcc fx_carry(FxAcc r) {
+    r.h = fx_add32((int)fx_u1(r.c), r.h);
+    r.c = (fx)fx_u0(r.c);
+    FX_TRACK(r.most = 0x1p32;)
     return r;
 }
 FX_HD bool fx_fits(fx a, int s) { return s < 64 && (fx)((ufx)a << s) >> s == a; }
@@ -382,7 +397,7 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
         FxAcc s = fx_mul(ww, X0);
         s = fx_mac(s, sg2w, Y);
         o.RK = mulk<3>(R1, k1);                    // Q60
-        s = fx_mac(s, sg + (w >> 1), o.RK);        // Q61 x Q60
+        s = fx_mac(fx_carry(s), sg + (w >> 1), o.RK);  // Q61 x Q60
         o.s0 = fx_sum<1>(s);                       // Q58
         FxAcc e = fx_mul(mulk<5>(ntw, v2), (P >> 1) - S);  // 2 () in Q60 x Q60
         e = fx_mac(e, nbw, o.s0);                          // Q62 x Q58; both doubled below
@@ -391,7 +406,7 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     {
         FxAcc s = fx_mul(wt2, mulk<3>(dl, X0));            // Q62 x Q59
         s = fx_mac(s, mulk<3>(q.w, dl - sg), Y);           // 2 w~ (delta - sigma) in Q61 x Q60
-        s = fx_mac(s, dl - fx_shl(sg, 1), Q);              // -(2 sigma - delta) Q61 x Q60
+        s = fx_mac(fx_carry(s), dl - fx_shl(sg, 1), Q);    // -(2 sigma - delta) Q61 x Q60
         o.s1 = fx_sum<1>(s);                               // Q58
         FxAcc e = fx_mul(nbw, o.s1);                       // Q62 x Q58
         e = fx_mac(e, nigk1, wP);                          // Q60 x 2 w~ P in Q60

@@ -1,10 +1,11 @@
 """The number ranges of the fixed-point geodesic (csrc/fixed_geodesic.cuh) on
 the CPU: a build in which every product, shift and sum that loses bits of its
 value, and every shift by a word's length or more (which differs between
-machines), ends the program, over both ends of the grids' range and views from
-the polar axis to the equator.  A product that wraps is off by its format's
-range, and the ray by 1e-4 or far more: its final state is held to 1e-7 of
-long double."""
+machines), ends the program, and so does a sum of products whose cross terms
+could come to more than 64 bits, over both ends of the grids' range and views
+from the polar axis to the equator.  A product that wraps is off by its
+format's range, and the ray by 1e-4 or far more: its final state is held to
+1e-7 of long double."""
 import os
 import subprocess
 
@@ -32,3 +33,15 @@ def test_no_bits_are_lost(check, hslope, inclination):
         assert run.returncode == 0, "an operation lost bits of its value"
         worst = float(run.stdout.split()[13])
         assert worst <= 1e-7, worst
+
+
+@pytest.mark.parametrize("case", ["150 0.02 2 0.9999 0.37148528972428885 177.03208629875422 40 836910",
+                                  "300 0.02 2 0.9999 0.2 4.903135877080161 40 577980",
+                                  "300 0.02 4 0.9999 1.8 1.3047726026769095 40 364885"])
+def test_no_ray_jumps(check, case):
+    """Rays that wind long close to a fast hole, where the cross terms of three
+    products fill more than 64 bits: no ray is more than eight times as far
+    off as its double-precision counterpart (beyond 1e-13)."""
+    run = subprocess.run([check, *case.split()], capture_output=True, text=True)
+    assert run.returncode == 0, "an operation lost bits of its value"
+    assert float(run.stdout.split()[12]) <= 8.0
