@@ -549,6 +549,16 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
                 k1 = s.k1 + mulk<1>(b1, third);
                 k2 = s.k2 + mulk<1>(b2, third);
                 k3 = s.k3 + mulk<1>(b3, third);
+            } else {
+                // RK2's offsets lose half a unit each, which N steps would add
+                // up to N/2 units: a unit is given back at every other step
+                const fx unit = (s.k0 ^ s.k1) & 1;
+                x1 += unit;
+                x2 += unit;
+                k0 += unit;
+                k1 += unit;
+                k2 += 1;  // two floors
+                k3 += unit;
             }
             // a wave vector that doubled within the step may have left its range inside it
             go = go && ((ufx)(fx_abs(k0) | fx_abs(k1) | fx_abs(k2) | fx_abs(k3)) >> 62) == 0;

@@ -45,3 +45,13 @@ def test_no_ray_jumps(check, case):
     run = subprocess.run([check, *case.split()], capture_output=True, text=True)
     assert run.returncode == 0, "an operation lost bits of its value"
     assert float(run.stdout.split()[12]) <= 8.0
+
+
+@pytest.mark.parametrize("case", ["20 0.002 2 0.9375 0.3 60 40 7", "20 0.002 2 0.5 1.0 175 40 7"])
+def test_rk2_roundings_do_not_add_up(check, case):
+    """Thousands of midpoint steps: the root mean square error of every state
+    component is at most the double-precision one (or 2^-52)."""
+    run = subprocess.run([check, *case.split()], capture_output=True, text=True)
+    vals = list(map(float, run.stdout.split()))
+    for fixed, double in zip(vals[0:12:2], vals[1:12:2]):
+        assert fixed <= max(double, 2.0 ** -52), vals
