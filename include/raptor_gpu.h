@@ -52,8 +52,9 @@ extern "C" {
 
 /* arithmetic forms */
 #define RAPTOR_PREC_FP64 0  /* FP64 transfer, the geodesic at least as precise: 64-bit fixed point
-                               (56 to 61 fraction bits) where R0 = 0, 0.2 <= hslope <= 1.8 and
-                               0.02 <= stepsize <= 0.1 for every image of the call, else FP64 */
+                               (56 to 61 fraction bits) where R0 = 0, 0.2 <= hslope <= 1.8,
+                               0.02 <= stepsize <= 0.1 and the camera's x2 is 2^-13 or more from
+                               0 and 1 for every image of the call, else FP64 */
 #define RAPTOR_PREC_MIXED 1 /* geodesic as RAPTOR_PREC_FP64, FP32 fluid/emission/transfer */
 #define RAPTOR_PREC_MIXED_DF 2 /* geodesic + metric in double-float (pairs of FP32, 48-bit
                                   significand) on the FP32 pipes, transfer as RAPTOR_PREC_MIXED */

@@ -40,3 +40,17 @@ def test_axis_views_match_port(eng, hslope, inclination, integrator):
     for key in ("d_m_unit", "d_r_high", "d_r_low", "d_inclination"):
         scale = max(abs(g[key]), 1e-6 * abs(g["d_r_high"]))
         assert abs(m[key] - g[key]) <= 2e-3 * scale, (key, m[key], g[key])
+
+
+# hslope 0.3: the render's line at a camera x2 of 2^-13 lies at 0.037 degrees
+@pytest.mark.parametrize("inclination", [0.03, 0.05, 179.95, 179.97])
+def test_both_sides_of_the_renders_line(eng, torus64, inclination):
+    from oracle import port
+    from raptor_gb300 import engine
+    desc = engine.image_desc(24, 21, [230e9], grid=eng.upload_grid(torus64.geom, torus64.prims),
+                             inclination=inclination)
+    img, spec = eng.render(desc, engine.PREC_FP64)
+    ref = port.Scene(torus64.geom, torus64.prims, 24, 21, inclination=inclination).render([230e9])[0][:, 0]
+    assert_fp64_parity(img, ref, f"{inclination} degrees")
+    mixed, mspec = eng.render(desc, engine.PREC_MIXED)
+    assert abs(mspec[0] - spec[0]) <= FLUX_RTOL_MIXED * abs(spec[0])
