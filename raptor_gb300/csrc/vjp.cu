@@ -996,6 +996,14 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
         CK(cudaMemsetAsync(ctx->d_grad, 0, sizeof(double) * (4 + 3 * ncell), ctx->stream));
         CK(cudaMemsetAsync(ctx->d_counters, 0, kCtrCount * sizeof(unsigned long long), ctx->stream));
 
+        // The mixed adjoint steps in fixed point unless its camera is close to
+        // the axis: a step that falls back to FP64 carries its tangent there and
+        // costs more than one of vjp_kernel_mixed.  512x512 at five frequencies,
+        // hslope 0.3 (fixed point, FP64): 0.15 degrees 337, 226 ms; 0.5 degrees
+        // 239, 215; 0.8 degrees 211, 206; 17 degrees 86, 148.  hslope 1.8: 0.03
+        // degrees 270, 213; 0.06 degrees 227, 202.  2^-8 in x2 is 1.2 degrees at
+        // hslope 0.3 and 0.14 at 1.8.
+        const bool fixed = b.fixed && him.xcam[2] > 0x1p-8 && him.xcam[2] < 1.0 - 0x1p-8;
         // the adjoint of the form that rendered: FP64 duals for the FP64 form;
         // for the mixed and mixed-DF forms their own geodesic with FP32
         // tangents and the FP32 dual sample (vjp_df.cu)
@@ -1005,7 +1013,7 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
         const VjpLaunchFn vfn =
             precision == RAPTOR_PREC_MIXED_DF ? pick_vjp_df(b.max_nf, &kp, kappa, one_pass)
             : precision == RAPTOR_PREC_MIXED
-                ? (b.fixed ? pick_vjp_fx : pick_vjp_mixed)(b.max_nf, &kp, kappa, one_pass)
+                ? (fixed ? pick_vjp_fx : pick_vjp_mixed)(b.max_nf, &kp, kappa, one_pass)
                 : pick_vjp_fp64(b.max_nf, &kp, !ctx->opt.no_sample_pool, &scratch_rows, kappa, one_pass);
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kp, kVjpBlock, 0));
         // The pooled FP64 adjoint takes one block per SM up to five rays per lane

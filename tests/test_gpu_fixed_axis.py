@@ -54,3 +54,22 @@ def test_both_sides_of_the_renders_line(eng, torus64, inclination):
     assert_fp64_parity(img, ref, f"{inclination} degrees")
     mixed, mspec = eng.render(desc, engine.PREC_MIXED)
     assert abs(mspec[0] - spec[0]) <= FLUX_RTOL_MIXED * abs(spec[0])
+
+
+# and the mixed adjoint's, of 2^-8, at 1.2 degrees
+@pytest.mark.parametrize("tape", [0, -1], ids=["one_pass", "two_passes"])
+@pytest.mark.parametrize("inclination", [1.1, 1.3, 178.7, 178.9])
+def test_both_sides_of_the_adjoints_line(torus64, inclination, tape):
+    from raptor_gb300 import engine
+    e = engine.Engine(vjp_tape=tape)
+    desc = engine.image_desc(32, 31, [230e9], grid=e.upload_grid(torus64.geom, torus64.prims),
+                             inclination=inclination, m_unit=1e19)
+    img, _ = e.render(desc, engine.PREC_FP64)
+    w = img / np.sum(img * img)
+    _, g = e.vjp(desc, w, engine.PREC_FP64)
+    out, m = e.vjp(desc, w, engine.PREC_MIXED)
+    e.close()
+    assert np.max(np.abs(out - img)) <= 1e-3 * np.max(img)
+    for key in ("d_m_unit", "d_r_high", "d_r_low", "d_inclination"):
+        scale = max(abs(g[key]), 1e-6 * abs(g["d_r_high"]))
+        assert abs(m[key] - g[key]) <= 2e-3 * scale, (key, m[key], g[key])
