@@ -564,9 +564,17 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
 // 210x211 mixed 15.4 -> 17.1).  The FP64 form's samples keep more warps busy:
 // up to 3/2 (128x128 13.2 -> 12.5, 140x141 at three frequencies 17.2 -> 15.5;
 // 190x191 14.8 -> 15.6).
+// Where the geodesic is FP64 (not fast), its pipe is what a launch waits for,
+// four warps per SM keep it busy, and the queue then deals the rays evenly
+// over the SMs; with three blocks some SMs hold twice the others' share, which
+// ones being a matter of how the blocks arrive.  Up to five rays per lane
+// (median and spread of 12 runs at all the blocks that fit, at one): mixed
+// 86x161 48.2 (35-55), 31.9 (31.8-32.0) ms; 190x191 40.5, 27.1; 320x321 at five
+// frequencies 62.1, 52.8; FP64 128x127 50.8 (44-56), 41.2; 220x221 44.8, 35.5;
+// 320x321 at five 74.1, 74.6.
 int default_blocks(int form, bool fast, long long rays, int sms, int block, int occ) {
     const long long lanes = (long long)sms * block;
-    return fast && rays * 2 <= lanes * (form == RAPTOR_PREC_FP64 ? 3 : 4) ? 1 : occ;
+    return rays * 2 <= lanes * (!fast ? 10 : form == RAPTOR_PREC_FP64 ? 3 : 4) ? 1 : occ;
 }
 
 LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, long long rays) {

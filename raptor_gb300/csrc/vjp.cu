@@ -1016,14 +1016,17 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
                 ? (fixed ? pick_vjp_fx : pick_vjp_mixed)(b.max_nf, &kp, kappa, one_pass)
                 : pick_vjp_fp64(b.max_nf, &kp, !ctx->opt.no_sample_pool, &scratch_rows, kappa, one_pass);
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kp, kVjpBlock, 0));
-        // The pooled FP64 adjoint takes one block per SM up to five rays per lane
-        // of such a launch: the queue then deals the rays evenly, where eight
-        // warps per SM leave some SMs twice the others' share of the FP64 pipe's
-        // work, and four keep that pipe as busy.  128x128 83 -> 65 ms (and 15 %
-        // from run to run -> 1 %), 256x255 126 -> 107, 300x301 152 -> 141;
-        // 340x341 and above within 2 % either way.
-        const bool even = precision == RAPTOR_PREC_FP64 && !ctx->opt.no_sample_pool &&
-                          re - rb <= 5ll * ctx->num_sms * kVjpBlock;
+        // The adjoints whose geodesic is FP64 take one block per SM up to five
+        // rays per lane of such a launch, the mixed one up to 5/2: the queue then
+        // deals the rays evenly, where eight warps per SM leave some SMs twice the
+        // others' share of the FP64 pipe's work (which ones being a matter of how
+        // the blocks arrive), and four keep that pipe as busy.  Median and spread
+        // of 9 runs at two blocks and at one: FP64 in place 54x69 at five
+        // frequencies 122 (113-131), 82 (81-83) ms; 128x127 158, 128; 300x301 at
+        // five 223, 207; mixed 160x161 at two 41.9, 34.4; 220x221 47.2, 38.8;
+        // 270x271 RK2 28.0, 31.7.
+        const long long most = fp64 ? 10 : precision == RAPTOR_PREC_MIXED && !fixed ? 5 : 0;
+        const bool even = 2 * (re - rb) <= most * ctx->num_sms * kVjpBlock;
         const int grid = ctx->num_sms * (even ? 1 : std::max(occ, 1));
         // the pooled adjoint's per-warp result slices (several frequencies)
         if (scratch_rows > 0) {

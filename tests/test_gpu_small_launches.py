@@ -1,0 +1,65 @@
+"""Launches of few rays whose geodesic is FP64 (here: R0 just off 0) take one
+block per SM, and the shape changes no bit of a render."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.fixture(scope="module")
+def off_zero(torus64):
+    return dataclasses.replace(torus64.geom, R0=1e-12), torus64.prims
+
+
+def _size(rays):
+    """The largest image of height 128 with at most this many rays, and one more column."""
+    return (rays // 128, 128), (rays // 128 + 1, 128)
+
+
+@pytest.mark.parametrize("prec,opts", [(0, {}), (0, {"no_sample_pool": 1}), (1, {})], ids=["pool", "in_place", "mixed"])
+def test_renders_at_both_sides_of_the_line(off_zero, prec, opts):
+    from raptor_gb300 import engine
+    inside, outside = _size(5 * 128 * _sms())
+    eng, ref = engine.Engine(**opts), engine.Engine(blocks_per_sm=2, **opts)
+    ga, gb = eng.upload_grid(*off_zero), ref.upload_grid(*off_zero)
+    for (w, h), one in ((inside, True), (outside, False)):
+        kw = dict(stepsize=0.1, integrator=2)
+        a, _ = eng.render(engine.image_desc(w, h, [230e9], grid=ga, **kw), prec)
+        assert (eng.stats()["blocks_per_sm"] == 1) == one
+        b, _ = ref.render(engine.image_desc(w, h, [230e9], grid=gb, **kw), prec)
+        assert ref.stats()["blocks_per_sm"] == 2
+        assert np.array_equal(a, b) and np.any(a)
+    eng.close()
+    ref.close()
+
+
+@pytest.mark.parametrize("prec,opts,rays_per_lane", [(0, {}, 5), (0, {"no_sample_pool": 1}, 5), (1, {}, 2.5)],
+                         ids=["pool", "in_place", "mixed"])
+def test_adjoints_at_both_sides_of_the_line(off_zero, prec, opts, rays_per_lane):
+    """A launch just beyond the line and its halves, both within it: the
+    gradients are the halves' sums to the order of the sums (1e-12 in FP64;
+    1e-5, some hundred roundings, in the FP32 transfer's)."""
+    from raptor_gb300 import engine
+    eng = engine.Engine(**opts)
+    (w, h), (w1, _) = _size(int(rays_per_lane * 128 * _sms()))
+    kw = dict(grid=eng.upload_grid(*off_zero), stepsize=0.1, integrator=2)
+    tight = engine.image_desc(w, h, [230e9], **kw)
+    eng.vjp(tight, np.ones(w * h), prec, want_fields=False)
+    assert eng.stats()["grid_blocks"] == _sms()
+    desc, n = engine.image_desc(w1, h, [230e9], **kw), w1 * h
+    _, g = eng.vjp(desc, np.ones(n), prec, want_fields=False)
+    assert eng.stats()["grid_blocks"] > _sms()
+    _, lo = eng.vjp(desc, np.ones(n), prec, want_fields=False, ray_begin=0, ray_count=n // 2)
+    assert eng.stats()["grid_blocks"] == _sms()
+    _, hi = eng.vjp(desc, np.ones(n), prec, want_fields=False, ray_begin=n // 2, ray_count=n)
+    eng.close()
+    for key in ("d_m_unit", "d_r_high", "d_r_low", "d_inclination"):
+        parts = abs(lo[key]) + abs(hi[key])
+        assert abs(lo[key] + hi[key] - g[key]) <= (1e-12 if prec == 0 else 1e-5) * parts, key
