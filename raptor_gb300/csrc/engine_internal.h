@@ -41,6 +41,7 @@ struct Batch {
     long long total_rays = 0, out_len = 0;
     int spec_len = 0, max_nf = 1;
     bool fixed = false;  // every image is one the fixed-point geodesic covers (FxGeo::ok)
+    bool rk2 = false;    // an image takes the midpoint integrator
     size_t h2d_bytes = 0;
     std::vector<raptor::DevImage> host;
     std::vector<int> spec_img, spec_f;
@@ -100,8 +101,8 @@ RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool f
 RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool, long long rays);
 RayLaunchFn pick_ray_kernel_df(int nf, const void** fn, long long rays);
 // blocks per SM of a launch that names none
-int default_blocks(int form, bool fast, long long rays, int sms, int block, int occ);
-LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, long long rays);
+int default_blocks(int form, bool fast, bool rk2, long long rays, int sms, int block, int occ);
+LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, bool rk2, long long rays);
 LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp);
 int enqueue_render(raptor_gpu_ctx* ctx, const Batch& b, int form, long long rb, long long re,
                    const LaunchShape& ls, RayLaunchFn fn, bool timed, raptor::TraceSpec tr = {-1, nullptr, 0});

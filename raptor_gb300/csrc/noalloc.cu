@@ -189,7 +189,7 @@ extern "C" int raptor_gpu_render_noalloc(int device, const double* d_cells, cons
         return RAPTOR_ERR_CUDA;
     LaunchShape ls;
     ls.block = kRayMaxBlock;
-    ls.bps = default_blocks(RAPTOR_PREC_FP64, fixed, rays, sms, ls.block, occ > 0 ? occ : 1);
+    ls.bps = default_blocks(RAPTOR_PREC_FP64, fixed, false, rays, sms, ls.block, occ > 0 ? occ : 1);
     ls.grid = sms * ls.bps;
     ls.refill = fixed ? kDefaultRefillFast : kDefaultRefill;
     fn(ls, st, d_desc, n_imgs, 0, rays, d_ctr, d_I_out, TraceSpec{-1, nullptr, 0});

@@ -504,6 +504,7 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
     b.spec_len = 0;
     b.max_nf = 1;
     b.fixed = true;
+    b.rk2 = false;
     b.host.resize(n_imgs);
     b.spec_img.clear();
     b.spec_f.clear();
@@ -511,6 +512,7 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
         int rc = build_dev_image(ctx, imgs[k], b.host[k]);
         if (rc) return rc;
         b.fixed = b.fixed && b.host[k].fx.ok;
+        b.rk2 = b.rk2 || b.host[k].integrator == RAPTOR_RK2;
         b.host[k].ray_begin = b.total_rays;
         b.host[k].out_offset = b.out_len;
         b.total_rays += (long long)imgs[k].width * imgs[k].height;
@@ -572,12 +574,17 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
 // 86x161 48.2 (35-55), 31.9 (31.8-32.0) ms; 190x191 40.5, 27.1; 320x321 at five
 // frequencies 62.1, 52.8; FP64 128x127 50.8 (44-56), 41.2; 220x221 44.8, 35.5;
 // 320x321 at five 74.1, 74.6.
-int default_blocks(int form, bool fast, long long rays, int sms, int block, int occ) {
+// The double-float kernels hide a midpoint step's shorter chains worse: with it
+// only up to one ray per lane (30,000 to 36,000 rays, one and two blocks: five
+// images of a 15 M field at steps of 0.02 23.2, 17.9 ms; 190x191 at 0.015 20.9,
+// 17.9; at three frequencies and 0.05 8.4, 7.9).
+int default_blocks(int form, bool fast, bool rk2, long long rays, int sms, int block, int occ) {
     const long long lanes = (long long)sms * block;
-    return rays * 2 <= lanes * (!fast ? 10 : form == RAPTOR_PREC_FP64 ? 3 : 4) ? 1 : occ;
+    const int halves = form == RAPTOR_PREC_MIXED_DF ? (rk2 ? 2 : 4) : !fast ? 10 : form == RAPTOR_PREC_FP64 ? 3 : 4;
+    return rays * 2 <= lanes * halves ? 1 : occ;
 }
 
-LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, long long rays) {
+LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, bool rk2, long long rays) {
     const bool fast = form == RAPTOR_PREC_MIXED_DF || fixed;
     LaunchShape ls;
     ls.block = ctx->opt.block_size > 0 ? ctx->opt.block_size : kRayMaxBlock;
@@ -586,7 +593,7 @@ LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fi
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, ls.block, 0);
     occ = std::max(occ, 1);
     int bps = ctx->opt.blocks_per_sm > 0 ? std::min(ctx->opt.blocks_per_sm, occ)
-                                         : default_blocks(form, fast, rays, ctx->num_sms, ls.block, occ);
+                                         : default_blocks(form, fast, rk2, rays, ctx->num_sms, ls.block, occ);
     ls.grid = ctx->num_sms * bps;
     ls.bps = bps;
     ls.refill = ctx->opt.refill_interval > 0 ? ctx->opt.refill_interval
@@ -789,7 +796,7 @@ extern "C" int raptor_gpu_trace_ray(raptor_gpu_ctx* ctx, const raptor_image_desc
     CK(cudaMemsetAsync(ctx->d_trace, 0, bytes, ctx->stream));
     const void* fnp = nullptr;
     RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, false, false, 1);  // the trace kernels step in FP64
-    LaunchShape ls = default_shape(ctx, fnp, precision, false, 1);
+    LaunchShape ls = default_shape(ctx, fnp, precision, false, false, 1);
     ls.grid = 1;
     ls.block = 32;
     TraceSpec tr{pixel, ctx->d_trace, max_records};

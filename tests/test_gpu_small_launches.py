@@ -1,5 +1,6 @@
-"""Launches of few rays whose geodesic is FP64 (here: R0 just off 0) take one
-block per SM, and the shape changes no bit of a render."""
+"""Launches of few rays take one block per SM, and the shape changes no bit of
+a render: the kernels whose geodesic is FP64 (here: R0 just off 0) and the
+double-float ones."""
 import dataclasses
 
 import numpy as np
@@ -63,3 +64,19 @@ def test_adjoints_at_both_sides_of_the_line(off_zero, prec, opts, rays_per_lane)
     for key in ("d_m_unit", "d_r_high", "d_r_low", "d_inclination"):
         parts = abs(lo[key]) + abs(hi[key])
         assert abs(lo[key] + hi[key] - g[key]) <= (1e-12 if prec == 0 else 1e-5) * parts, key
+
+
+@pytest.mark.parametrize("integrator,rays_per_lane", [(4, 2), (2, 1)], ids=["rk4", "rk2"])
+def test_double_float_lines(torus64, integrator, rays_per_lane):
+    from raptor_gb300 import engine
+    inside, outside = _size(rays_per_lane * 128 * _sms())
+    eng, ref = engine.Engine(), engine.Engine(blocks_per_sm=2)
+    ga, gb = (e.upload_grid(torus64.geom, torus64.prims) for e in (eng, ref))
+    for (w, h), one in ((inside, True), (outside, False)):
+        kw = dict(stepsize=0.1, integrator=integrator)
+        a, _ = eng.render(engine.image_desc(w, h, [230e9], grid=ga, **kw), engine.PREC_MIXED_DF)
+        assert (eng.stats()["blocks_per_sm"] == 1) == one
+        b, _ = ref.render(engine.image_desc(w, h, [230e9], grid=gb, **kw), engine.PREC_MIXED_DF)
+        assert np.array_equal(a, b) and np.any(a)
+    eng.close()
+    ref.close()
