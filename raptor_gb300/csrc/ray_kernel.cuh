@@ -46,10 +46,14 @@ enum : int {
 // 69.0 -> 70.0 ms).  With all or nearly all rays in flight at once the order
 // only gathers the long ones on the same SMs (mixed-DF 100x100 5.5 -> 6.0 ms,
 // 256x256 8.3 -> 8.8): they keep theirs.
+constexpr int kOrderedLanes = 8;
+__host__ __device__ __forceinline__ bool middle_out(long long n, long long lanes) {
+    return n * 4 > lanes * 5 && n <= lanes * kOrderedLanes;
+}
 __device__ __forceinline__ long long queue_order(unsigned long long idx, long long n) {
     const long long blocks = n >> 5, j = (long long)(idx >> 5);
-    const long long lanes = (long long)gridDim.x * blockDim.x;
-    if (j >= blocks || n * 4 <= lanes * 5 || n > lanes * 8) return (long long)idx;  // (the last, partial block keeps its place)
+    // (the last, partial block keeps its place)
+    if (j >= blocks || !middle_out(n, (long long)gridDim.x * blockDim.x)) return (long long)idx;
     const long long h = (j + 1) >> 1;
     return ((((blocks - 1) >> 1) + ((j & 1) ? h : -h)) << 5) | (long long)(idx & 31);
 }

@@ -27,7 +27,17 @@ using raptor::TraceSpec;
 
 namespace {
 
-std::string signature(const raptor_gpu_ctx* ctx, const Batch& b, int form) {
+int occupancy(const void* fn, int block) {
+    int occ = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, 0);
+    return std::max(occ, 1);
+}
+
+// What a tuned shape is kept for: the form, the size class, and what the rules
+// on the number of rays, whose lines lie inside the classes, make of it: the
+// kernel's blocks per SM (its register budget), one block per SM or all that
+// fit, and the queue's order.
+std::string signature(const raptor_gpu_ctx* ctx, const Batch& b, int form, const void* fnp, const LaunchShape& base) {
     char k[384];
     const int size_class = (int)std::log2((double)std::max<long long>(b.total_rays, 1));
     const char* name = form == RAPTOR_PREC_MIXED_DF ? "mixed_df"
@@ -35,7 +45,10 @@ std::string signature(const raptor_gpu_ctx* ctx, const Batch& b, int form) {
                        : ctx->opt.no_sample_pool    ? "fp64_inplace"
                                                     : "fp64";
     const char* geo = b.fixed && form != RAPTOR_PREC_MIXED_DF ? "_fx" : "";
-    snprintf(k, sizeof k, "%s|%s%s|nf%d|2^%d", ctx->device_name, name, geo, b.max_nf, size_class);
+    const char* grid = base.bps == 1 ? "one" : "full";
+    const char* order = raptor::middle_out(b.total_rays, (long long)base.grid * base.block) ? "middle" : "rows";
+    snprintf(k, sizeof k, "%s|%s%s|b%d|%s|%s|nf%d|2^%d", ctx->device_name, name, geo, occupancy(fnp, raptor::kRayMaxBlock),
+             grid, order, b.max_nf, size_class);
     std::string s(k);
     for (char& c : s)
         if (c == ' ') c = '_';
@@ -69,13 +82,11 @@ LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunc
     LaunchShape base = default_shape(ctx, fnp, form, b.fixed, b.rk2, b.total_rays);
     if (!ctx->opt.autotune) return base;
     load_file_cache(ctx);
-    const std::string key = signature(ctx, b, form);
+    const std::string key = signature(ctx, b, form, fnp, base);
     auto it = ctx->tuned.find(key);
     if (it != ctx->tuned.end()) {
         LaunchShape ls = it->second;
-        int occ = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fnp, ls.block, 0);
-        ls.bps = std::max(1, std::min(ls.bps, occ));
+        ls.bps = std::max(1, std::min(ls.bps, occupancy(fnp, ls.block)));
         ls.grid = ctx->num_sms * ls.bps;
         return ls;
     }
@@ -86,9 +97,7 @@ LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunc
     // interval are tuned.
     std::vector<LaunchShape> cands;
     for (int block : {64, 128}) {
-        int occ = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fnp, block, 0);
-        occ = std::max(occ, 1);
+        const int occ = occupancy(fnp, block);
         for (int refill : {1, 4, 8, 16}) {
             LaunchShape ls;
             ls.block = block;
