@@ -108,8 +108,11 @@ LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunc
         }
     }
     if (base.bps == 1) cands.push_back(base);  // a launch of all its rays at once (default_blocks)
-    const long long lanes = (long long)ctx->num_sms * 3 * 128;
-    const long long n = std::min<long long>(b.total_rays, 6 * lanes);
+    // the timed sample: a launch whose rays go in the order of rows is timed on
+    // enough of them to be one too, at every candidate's grid
+    long long lanes = 0;
+    for (const LaunchShape& ls : cands) lanes = std::max(lanes, (long long)ls.grid * ls.block);
+    const long long n = std::min<long long>(b.total_rays, (raptor::kOrderedLanes + 1) * lanes);
     const long long rb = (b.total_rays - n) / 2, re = rb + n;
     LaunchShape best = base;
     float best_ms = 1e30f;
