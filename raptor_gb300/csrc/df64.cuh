@@ -70,9 +70,10 @@ __device__ __forceinline__ DF add_f(DF a, float b) {
 }
 __device__ __forceinline__ DF operator-(DF a, DF b) { return a + (-b); }
 // The same sums where |a| >= |b|: Dekker's fast two-sum has the same exact
-// error in 3 operations instead of 6.  (Were the order broken, it would be off
-// by an ulp of the lo part's scale.)  1024x1024 69.1 -> 68.2 ms, its
-// 512x512 five-frequency VJP 52.5 -> 51.6, with the scaled sums below.
+// error in 3 operations instead of 6.  (Were b the larger by much, up to half an
+// ulp of the sum, all of the lo part, would be lost: each use states why it is
+// not.)  1024x1024 69.1 -> 68.2 ms, its 512x512 five-frequency VJP 52.5 -> 51.6,
+// with the scaled sums below.
 __device__ __forceinline__ DF add_ordered(DF a, DF b) {
     const DF s = quick_two_sum(a.hi, b.hi);
     return DF{s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo))};

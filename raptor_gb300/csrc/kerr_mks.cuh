@@ -93,7 +93,8 @@ __device__ __forceinline__ void mks_point_rolled(R x1, R x2, const G& g, MksPoin
         if (k == 1) break;
         p.s2x = sv;
         p.c2x = cv;
-        // theta = pi x2 + (1-h)/2 sin(2 pi x2) (metric.c:98), as theta / pi
+        // theta = pi x2 + (1-h)/2 sin(2 pi x2) (metric.c:98), as theta / pi; the
+        // second term is the smaller for 0 <= h <= 2
         arg = fma_small(g.th_coef, sv, x2);
     }
     p.s = sv;
@@ -119,12 +120,14 @@ __device__ __forceinline__ void geodesic_accel(const MksPointT<R>& p, const G& g
     const R s2th = 2.0 * sc;
     const R cot = c * p.isn;
     const R Sg = p.Sg, Sg2 = Sg * Sg;
-    const R r2a2 = add_ordered(r2, a2);  // r > 1 >= a outside the horizon
+    // outside the horizon r > 1 >= a; rays end before it unless R0 is below
+    // -r+/10, and then pile up there
+    const R r2a2 = add_ordered(r2, a2);
     const R two_r = 2.0 * r;
     const R Dl = add_ordered(r2a2, -two_r);  // Delta > 0
     const R Rr2 = two_r * r2a2;  // 2 r (r^2 + a^2)
     const R iS = p.iS, iS2 = iS * iS, iS3 = iS2 * iS;
-    const R B = add_ordered(2.0 * r2, -Sg) * iS3;
+    const R B = add_ordered(2.0 * r2, -Sg) * iS3;  // Sigma <= r^2 + a^2
     const R riS = r * iS;
     const R as2 = a * s2;
     const R aB = a * B;
