@@ -96,14 +96,14 @@ int prepare_batch(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n_imgs
 // form: RAPTOR_PREC_FP64, RAPTOR_PREC_MIXED or RAPTOR_PREC_MIXED_DF
 // pool: the FP64 form's sample-pool kernel (ray_kernel_pool) instead of ray_kernel
 // fixed: the fixed-point geodesic's kernels (FP64 and mixed forms; Batch::fixed)
-// rays: how many the batch has
+// rays: how many the launch has
 RayLaunchFn pick_ray_kernel(int nf, int form, const void** fn, bool pool, bool fixed, long long rays);
 RayLaunchFn pick_ray_kernel_fx(int nf, bool mixed, const void** fn, bool pool, long long rays);
 RayLaunchFn pick_ray_kernel_df(int nf, const void** fn, long long rays);
 // blocks per SM of a launch that names none
 int default_blocks(int form, bool fast, bool rk2, long long rays, int sms, int block, int occ);
 LaunchShape default_shape(raptor_gpu_ctx* ctx, const void* fn, int form, bool fixed, bool rk2, long long rays);
-LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp);
+LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp, long long rays);
 int enqueue_render(raptor_gpu_ctx* ctx, const Batch& b, int form, long long rb, long long re,
                    const LaunchShape& ls, RayLaunchFn fn, bool timed, raptor::TraceSpec tr = {-1, nullptr, 0});
 int collect_stats(raptor_gpu_ctx* ctx, bool timed);

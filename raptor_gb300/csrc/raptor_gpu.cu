@@ -728,9 +728,8 @@ static int render_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* imgs, int n
     if (rb > b.total_rays) return ctx_fail(ctx, RAPTOR_ERR_INVALID, "ray range starts past the batch");
     const int form = precision;
     const void* fnp = nullptr;
-    RayLaunchFn fn = pick_ray_kernel(b.max_nf, form, &fnp, !ctx->opt.no_sample_pool, b.fixed,
-                                     b.total_rays);
-    LaunchShape ls = choose_shape(ctx, b, form, fn, fnp);
+    RayLaunchFn fn = pick_ray_kernel(b.max_nf, form, &fnp, !ctx->opt.no_sample_pool, b.fixed, re - rb);
+    LaunchShape ls = choose_shape(ctx, b, form, fn, fnp, re - rb);
     bool replayed = false;
     if (ctx->opt.use_graph && rb == 0 && re == b.total_rays) {
         rc = graph_render(ctx, b, form, ls, fn, &replayed);

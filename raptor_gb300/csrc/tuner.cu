@@ -37,16 +37,17 @@ int occupancy(const void* fn, int block) {
 // on the number of rays, whose lines lie inside the classes, make of it: the
 // kernel's blocks per SM (its register budget), one block per SM or all that
 // fit, and the queue's order.
-std::string signature(const raptor_gpu_ctx* ctx, const Batch& b, int form, const void* fnp, const LaunchShape& base) {
+std::string signature(const raptor_gpu_ctx* ctx, const Batch& b, int form, const void* fnp, const LaunchShape& base,
+                      long long rays) {
     char k[384];
-    const int size_class = (int)std::log2((double)std::max<long long>(b.total_rays, 1));
+    const int size_class = (int)std::log2((double)std::max<long long>(rays, 1));
     const char* name = form == RAPTOR_PREC_MIXED_DF ? "mixed_df"
                        : form == RAPTOR_PREC_MIXED  ? "mixed"
                        : ctx->opt.no_sample_pool    ? "fp64_inplace"
                                                     : "fp64";
     const char* geo = b.fixed && form != RAPTOR_PREC_MIXED_DF ? "_fx" : "";
     const char* grid = base.bps == 1 ? "one" : "full";
-    const char* order = raptor::middle_out(b.total_rays, (long long)base.grid * base.block) ? "middle" : "rows";
+    const char* order = raptor::middle_out(rays, (long long)base.grid * base.block) ? "middle" : "rows";
     snprintf(k, sizeof k, "%s|%s%s|b%d|%s|%s|nf%d|2^%d", ctx->device_name, name, geo, occupancy(fnp, raptor::kRayMaxBlock),
              grid, order, b.max_nf, size_class);
     std::string s(k);
@@ -78,11 +79,11 @@ void save_file_cache(const std::string& key, const LaunchShape& ls) {
 
 }  // namespace
 
-LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp) {
-    LaunchShape base = default_shape(ctx, fnp, form, b.fixed, b.rk2, b.total_rays);
+LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunchFn fn, const void* fnp, long long rays) {
+    LaunchShape base = default_shape(ctx, fnp, form, b.fixed, b.rk2, rays);
     if (!ctx->opt.autotune) return base;
     load_file_cache(ctx);
-    const std::string key = signature(ctx, b, form, fnp, base);
+    const std::string key = signature(ctx, b, form, fnp, base, rays);
     auto it = ctx->tuned.find(key);
     if (it != ctx->tuned.end()) {
         LaunchShape ls = it->second;
@@ -112,7 +113,7 @@ LaunchShape choose_shape(raptor_gpu_ctx* ctx, const Batch& b, int form, RayLaunc
     // enough of them to be one too, at every candidate's grid
     long long lanes = 0;
     for (const LaunchShape& ls : cands) lanes = std::max(lanes, (long long)ls.grid * ls.block);
-    const long long n = std::min<long long>(b.total_rays, (raptor::kOrderedLanes + 1) * lanes);
+    const long long n = std::min<long long>(rays, (raptor::kOrderedLanes + 1) * lanes);
     const long long rb = (b.total_rays - n) / 2, re = rb + n;
     LaunchShape best = base;
     float best_ms = 1e30f;

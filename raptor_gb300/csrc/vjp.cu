@@ -982,8 +982,8 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
         if (!one_pass) {
             const void* fnp = nullptr;
             RayLaunchFn fn = pick_ray_kernel(b.max_nf, precision, &fnp, !ctx->opt.no_sample_pool, b.fixed,
-                                             b.total_rays);
-            LaunchShape ls = choose_shape(ctx, b, precision, fn, fnp);
+                                             re - rb);
+            LaunchShape ls = choose_shape(ctx, b, precision, fn, fnp, re - rb);
             rc = enqueue_render(ctx, b, precision, rb, re, ls, fn, true);
             if (rc) return rc;
             CK(cudaMemcpyAsync(fwd_ctr, ctx->d_counters, sizeof fwd_ctr, cudaMemcpyDeviceToHost, ctx->stream));
