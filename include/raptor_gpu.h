@@ -229,7 +229,7 @@ int raptor_gpu_trace_ray(raptor_gpu_ctx *ctx, const raptor_image_desc *img, int 
  * (may be NULL) then receives the image that pass renders, equal to
  * raptor_gpu_render's to rounding (in FP64, whose adjoint steps the geodesic
  * in FP64, 1e-11 of the largest pixel but for rays that circle the hole, which
- * amplify it to 1e-9; 1e-5 with the FP32 transfers).  In two passes (vjp_tape = -1, the in-place FP64
+ * amplify it to 1e-8; 1e-5 with the FP32 transfers).  In two passes (vjp_tape = -1, the in-place FP64
  * adjoint, or a tape too small) the form's forward render runs first and
  * I_out receives it.
  * No counterpart in the reference, which has no derivatives. */

@@ -1082,7 +1082,8 @@ static int vjp_impl(raptor_gpu_ctx* ctx, const raptor_image_desc* img, int preci
         memset(&s, 0, sizeof s);
         s.kernel_ms = vjp_ms;
         s.device_ms = fwd_ms + vjp_ms;
-        // counters of the adjoint pass (the forward pass takes the same steps)
+        // counters of the adjoint pass (the forward pass takes the same steps; in
+        // FP64 its geodesic is the render's, which may be fixed point: to rounding)
         s.rays = (long long)ctr[kCtrRays];
         s.steps = (long long)ctr[kCtrSteps];
         s.rt_calls = (long long)ctr[kCtrRtCalls];

@@ -85,15 +85,18 @@ def test_double_float_lines(torus64, integrator, rays_per_lane):
 @pytest.mark.parametrize("prec", [0, 1, 2], ids=["fp64", "mixed", "mixed_df"])
 def test_a_range_takes_its_own_launch_rules(torus64, prec):
     """A small range of a large image is launched as a small image is, with the
-    bits of the whole."""
+    bits of the whole: every register budget of a form's kernel gives the same
+    (FP64: 4, 3 and 2 blocks per SM, the others 3 and 2)."""
     from raptor_gb300 import engine
     eng = engine.Engine()
     w, h = 1024, 4 * _sms()
     desc = engine.image_desc(w, h, [230e9], grid=eng.upload_grid(torus64.geom, torus64.prims), stepsize=0.1)
     full, _ = eng.render(desc, prec)
     assert eng.stats()["blocks_per_sm"] > 1
-    begin, count = w * h // 2 - 3000, 100 * _sms()
-    part, _ = eng.render(desc, prec, ray_begin=begin, ray_count=count)
-    assert eng.stats()["blocks_per_sm"] == 1 and eng.stats()["rays"] == count
-    assert np.array_equal(part[begin:begin + count], full[begin:begin + count]) and np.any(part)
+    for rays_per_sm, one in ((100, True), (400, False), (1000, False), (2000, False)):
+        count = rays_per_sm * _sms()
+        begin = (w * h - count) // 2
+        part, _ = eng.render(desc, prec, ray_begin=begin, ray_count=count)
+        assert (eng.stats()["blocks_per_sm"] == 1) == one and eng.stats()["rays"] == count
+        assert np.array_equal(part[begin:begin + count], full[begin:begin + count]) and np.any(part)
     eng.close()
