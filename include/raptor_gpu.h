@@ -54,7 +54,9 @@ extern "C" {
 #define RAPTOR_PREC_FP64 0  /* FP64 transfer, the geodesic at least as precise: 64-bit fixed point
                                (56 to 61 fraction bits) where R0 = 0, 0.2 <= hslope <= 1.8,
                                0.02 <= stepsize <= 0.1 and the camera's x2 is 2^-13 or more from
-                               0 and 1 for every image of the call, else FP64 */
+                               0 and 1 for every image of the call, else FP64 (one image out
+                               of range moves its whole batch there: slower, and the others'
+                               pixels differ in their last bits) */
 #define RAPTOR_PREC_MIXED 1 /* geodesic as RAPTOR_PREC_FP64, FP32 fluid/emission/transfer */
 #define RAPTOR_PREC_MIXED_DF 2 /* geodesic + metric in double-float (pairs of FP32, 48-bit
                                   significand) on the FP32 pipes, transfer as RAPTOR_PREC_MIXED */
@@ -212,7 +214,10 @@ int raptor_gpu_get_stats(const raptor_gpu_ctx *ctx, raptor_gpu_stats *out);
  * the initial photon): c = 0..7 photon_u, 8 d lambda, 9 tau of the first
  * frequency, 10 its intensity before the nu^3 scaling, 11 steps, 12 theta
  * turns, 13 event (0 no transfer, 1 sigma cut, 2 sampled, 3 escaped), 14 the
- * order-limit stop flag, 15 unused.  *n_records = records written. */
+ * order-limit stop flag, 15 unused.  *n_records = records written.  A trace
+ * of the FP64 or mixed form steps in FP64; where those render with the
+ * fixed-point geodesic (RAPTOR_PREC_FP64) the recorded path is the rendered
+ * one to rounding. */
 #define RAPTOR_TRACE_WIDTH 16
 int raptor_gpu_trace_ray(raptor_gpu_ctx *ctx, const raptor_image_desc *img, int precision, int pixel,
                          int max_records, double *records, int *n_records);

@@ -345,11 +345,11 @@ FX_HD fx fx_isigma(const FxGeo& g, const FxPoint& p, int n, fx& a2w2, fx& s2, fx
     return fx_recip(sg);                                // 2/sigma in Q61, the integer of 1/sigma in Q62
 }
 
-// The terms of a stage's right-hand side and the point, for a tangent of it.
+// The terms of a stage's right-hand side that a tangent of it reads.
 struct FxTerms {
-    fx w, ww, wt2, wt3, a2w2, s2, sg, isg, rho, dl, isg2, isg3, beta, gam, aw, sc, thi, t, as2;
-    fx P, R1, S, H, X0, Y, Q, RK, kap2, kap3, mu, s0, s1;
-    fx sg2, wr2, rww, F1, F2, z, A, g2, G, B, F3, D;
+    fx wt2, s2, sg, isg, rho, dl, isg2, isg3, beta, gam, sc, thi;
+    fx R1, S, H, X0, Y, RK, s0, s1;
+    fx sg2, F1, F2, z, g2, G, F3;
     fx E0, E1, E2a, E2b, E3a, E3b;
 };
 
@@ -418,12 +418,12 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
     const fx wr2 = mulk<2>(w, rho);                // 2 w rho in Q60
     const fx kv23 = mulk<5>(k2, v3);               // Q60
     {
-        o.rww = mulk<2>(rho, ww);                                                      // Q61
-        const fx F1 = fx_sum<1>(fx_mac(fx_mul(sg2 + wr2, k1), o.rww, k0));             // Q58
+        const fx rww = mulk<2>(rho, ww);                                               // Q61
+        const fx F1 = fx_sum<1>(fx_mac(fx_mul(sg2 + wr2, k1), rww, k0));               // Q58
         const fx F2 = fx_sum<3>(fx_mac(fx_mul(dl, sg2), wr2, rho));                    // Q60
         const fx z = mulk<3>(mulk<2>(sc, isg3), q.ithp);                               // Q62
-        o.A = mulk<3>(a2w2, wt3);                                   // 2 a^2 w^2 w~^3 2^-p in Q61
-        FxAcc e = fx_mul(o.A, mulk<1>(z, H));                       // x Q58
+        const fx A = mulk<3>(a2w2, wt3);                            // 2 a^2 w^2 w~^3 2^-p in Q61
+        FxAcc e = fx_mul(A, mulk<1>(z, H));                         // x Q58
         const fx g2 = mulk<3>(g.th2, mulk<3>(q.s2x, q.ithp));       // th''/th', Q59
         e = fx_mac(e, (t >> 1) - g2, mulk<5>(k2, v2));              // Q59 x Q60
         e = fx_mac(e, nigk1 >> 1, k2);                              // 2 () in Q58 x Q61
@@ -434,8 +434,8 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
         o.E2b = mulk<2>(fx_shl(z, q.ks), mulk<3>(k3, G));             // Q62 x Q57
     }
     {
-        o.B = mulk<2>(mulk<2>(g.a, nbw), wt3) >> u;                             // Q61
-        FxAcc e = fx_mul(o.B, H - mulk<2>(k0, P));                              // x (H - 2 K0 P) Q59
+        const fx B = mulk<2>(mulk<2>(g.a, nbw), wt3) >> u;                      // Q61
+        FxAcc e = fx_mul(B, H - mulk<2>(k0, P));                              // x (H - 2 K0 P) Q59
         e = fx_mac(e, mulk<1>(gam, k3), (wP >> 1) - k1);                        // Q60 x (w~ P - 2 K1) Q60
         e = fx_mac(e, ntw, kv23);                                               // 4 () in Q60 x Q60
         o.E3a = fx_sum<1>(e) + (mulk<1>(awt >> p, M2) >> (u + 1));              // a w kap2 th' K2/sigma: Q62 x Q59
@@ -443,13 +443,11 @@ FX_HD void fx_rhs(const FxGeo& g, const FxPoint& q, fx k0, fx k1, fx k2, fx k3, 
         const fx D = (mulk<2>(mulk<2>(aw, isg2), mulk<3>(k2, F3)) >> u) - kv23;  // Q60
         o.E3b = mulk<3>(mulk<2>(mulk<2>(q.c, q.isn), q.thp), D);                // -cot th' 2^-ks () Q59 x Q60
         o.F3 = F3;
-        o.D = D;
     }
     // (terms that nothing reads cost nothing: the function is inlined)
-    o.w = w; o.ww = ww; o.wt2 = wt2; o.wt3 = wt3; o.a2w2 = a2w2; o.s2 = s2; o.sg = sg; o.isg = isg;
-    o.rho = rho; o.dl = dl; o.isg2 = isg2; o.isg3 = isg3; o.beta = beta; o.gam = gam; o.aw = aw;
-    o.sc = sc; o.thi = thi; o.t = t; o.as2 = as2; o.P = P; o.R1 = R1; o.S = S; o.H = H; o.X0 = X0;
-    o.Y = Y; o.Q = Q; o.kap2 = kap2; o.kap3 = kap3; o.mu = mu; o.sg2 = sg2; o.wr2 = wr2;
+    o.wt2 = wt2; o.s2 = s2; o.sg = sg; o.isg = isg; o.rho = rho; o.dl = dl; o.isg2 = isg2; o.isg3 = isg3;
+    o.beta = beta; o.gam = gam; o.sc = sc; o.thi = thi; o.R1 = R1; o.S = S; o.H = H; o.X0 = X0; o.Y = Y;
+    o.sg2 = sg2;
 }
 
 FX_HD fx fx_vshift(fx k, int e) { return k >> (3 - e); }  // K 2^e in Q58, e <= 3

@@ -192,8 +192,9 @@ __device__ __forceinline__ bool fx_in_grid(const DevImage& im, const FxState& c)
 // 512x512 33.9, 36.0; 400x400 22.9, 23.3; 360x360 20.5, 19.8; 256x256 16.7,
 // 14.8; 128x128 11.7, 10.7; five frequencies 320x320 24.0, 20.2: kFxFewRaysMixed.
 // 5 blocks (96 registers) are slower throughout.
-// A barrier per step (kLockstep) keeps the four warps of a pooled block on the
-// same code: 1024x1024 214 -> 202 ms.
+// A barrier per step (kLockstep, which only the pooled kernel reads) keeps the
+// four warps of a block on the same code: 1024x1024 214 -> 202 ms.  The lines
+// between the kernels are numbers of rays on GB300's 152 SMs.
 constexpr long long kFxFewRays = 3ll << 15, kFxManyRays = 1ll << 19;
 constexpr long long kFxFewRaysMixed = 1ll << 17;
 

@@ -28,7 +28,7 @@ struct FxPointF1 {
 };
 __device__ __forceinline__ FxPointF1 fx_point_f1(const FxGeo& g, const FxPoint& q, int n, float d1, float d2) {
     const float r = fx_lead(q.r, exp2i(n - 29)), w = fx_lead(q.w, exp2i(-n - 30));
-        const float s = fx_lead(q.s, 0x1p-30f), c = fx_lead(q.c, 0x1p-30f);
+    const float s = fx_lead(q.s, 0x1p-30f), c = fx_lead(q.c, 0x1p-30f);
     const float thp = fx_lead(q.thp, 0x1p-28f), ithp = fx_lead(q.ithp, 0x1p-29f);
     const float isn = fx_lead(q.isn, exp2i(q.ks - 29));
     const float dthp = fx_lead(g.th2, 0x1p-26f) * fx_lead(q.s2x, 0x1p-30f);
@@ -110,7 +110,9 @@ struct FxTangent {
     }
     // stage q: the differentials of the terms o of fx_rhs (those of order one
     // from their leading words, the products that shrink with 1/r or the
-    // angular momentum formed in FP32), then of the offset h f (h = L/2, L/2, L, L/2; RK2 L/2, L)
+    // angular momentum formed in FP32: from the fixed-point terms instead,
+    // d_inclination is as far from the FP64 adjoint's, 2.8e-6 in the median
+    // view, and the pass 7 % slower), then of the offset h f (h = L/2, L/2, L, L/2; RK2 L/2, L)
     __device__ __forceinline__ void stage(int q, int end, const FxPoint& pt, const FxTerms& o, fx k0f, fx k1f, fx k2f,
                                           fx k3f) {
 #define Q(x, f) fx_lead(x, 0x1p32f / (float)(1ull << (f)))
