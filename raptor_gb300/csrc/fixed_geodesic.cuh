@@ -530,9 +530,13 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
     const int e = s.p - s.n;
     const fx full = -L, half = full >> 1;
     fx x1 = s.x1, x2 = s.x2, k0 = s.k0, k1 = s.k1, k2 = s.k2, k3 = s.k3;
+    // What symmetry keeps at exactly 0 has no products to round: k^3 of a ray in
+    // a plane through the axis of a hole without spin (which ends on the axis,
+    // and would pass it at a rounding's distance), k^2 in the equatorial plane.
+    const fx spins = (g.a | s.k3) != 0 ? 1 : 0, tilts = (s.k2 | (s.x2 - fx_one(61))) != 0 ? 1 : 0;
     // RK4's sums start at the mean of what the floors of their products lose
     // (p2 has two of them)
-    fx a1 = 0, a2 = 4, b0 = 4, b1 = 4, b2 = 6, b3 = 4;
+    fx a1 = 0, a2 = 4 * tilts, b0 = 4, b1 = 4, b2 = 6 * tilts, b3 = 4 * spins;
     const int end = rk2 ? 2 : 4;
 #ifdef __CUDACC__
 #pragma unroll 1
@@ -552,11 +556,11 @@ FX_HD void fx_step(const FxGeo& g, FxState& s, FxPoint& pt, bool rk2, double& dl
                 // up to N/2 units: a unit is given back at every other step
                 const fx unit = (s.k0 ^ s.k1) & 1;
                 x1 += unit;
-                x2 += unit;
+                x2 += unit & tilts;
                 k0 += unit;
                 k1 += unit;
-                k2 += 1;  // two floors
-                k3 += unit;
+                k2 += tilts;  // two floors
+                k3 += unit & spins;
             }
             // a wave vector that doubled within the step may have left its range inside it
             go = go && ((ufx)(fx_abs(k0) | fx_abs(k1) | fx_abs(k2) | fx_abs(k3)) >> 62) == 0;

@@ -55,3 +55,13 @@ def test_rk2_roundings_do_not_add_up(check, case):
     vals = list(map(float, run.stdout.split()))
     for fixed, double in zip(vals[0:12:2], vals[1:12:2]):
         assert fixed <= max(double, 2.0 ** -52), vals
+
+
+def test_symmetry_is_kept(tmp_path):
+    """Exact zeros of a ray's state stay exact: the sums' starts, which make up
+    for what floors lose on average, do not act where nothing is rounded."""
+    exe = str(tmp_path / "symmetry")
+    subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-x", "c++", "-o", exe,
+                    os.path.join(TESTS, "fixed_symmetry_check.cpp"), "-lm"], check=True)
+    steps = list(map(int, subprocess.run([exe], capture_output=True, text=True, check=True).stdout.split()))
+    assert len(steps) == 54 and min(steps) > 100, steps

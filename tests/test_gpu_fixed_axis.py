@@ -94,3 +94,22 @@ def test_mixed_inclination_gradient_over_views(eng):
         g, m = (eng.vjp(desc, w, p, want_fields=False)[1]["d_inclination"] for p in (0, 1))
         errors.append(abs(m / g - 1.0))
     assert np.median(errors) <= 1e-5, errors
+
+
+@pytest.mark.parametrize("size,inclination", [((33, 18), 20.0), ((33, 17), 90.0)])
+def test_axis_column_without_spin(eng, size, inclination):
+    """The middle column of an odd width looks along the axis.  Without spin its
+    rays' k^phi is 0 and they end on the axis at the step cap; they are counted
+    as in the FP64 geodesic (R0 of 1e-300, which changes no r), none non-finite."""
+    import dataclasses
+    from raptor_gb300 import engine, synth
+    d = synth.make_torus(n1=64, n2=64, a=0.0)
+    counts, images = [], []
+    for geom in (d.geom, dataclasses.replace(d.geom, R0=1e-300)):
+        desc = engine.image_desc(*size, [230e9], grid=eng.upload_grid(geom, d.prims), inclination=inclination)
+        with pytest.warns(engine.EngineWarning):
+            images.append(eng.render(desc, engine.PREC_FP64)[0])
+        st = eng.stats()
+        counts.append([st[k] for k in ("steps", "n_nonfinite", "n_stepcap")])
+    assert counts[0] == counts[1] and counts[0][1] == 0 and counts[0][2] > 0, counts
+    assert np.max(np.abs(images[0] - images[1])) <= 1e-9 * np.max(images[1])
